@@ -564,7 +564,8 @@ int fp::create_handle(int nx, int ny, int nz, double voxel_size, double mu, int 
     if (!fp::make_axis_plan(nx, P.px, err, P.stream) || !fp::make_axis_plan(ny, P.py, err, P.stream) ||
         !fp::make_axis_plan(nz, P.pz, err, P.stream))
         return fail(P, FP_ERR_UNSUPPORTED, err);
-    FP_CUDA(dalloc(P, reinterpret_cast<double2**>(&P.d_spec), 3 * (size_t)P.nh), "cudaMalloc spec");
+    FP_CUDA(dalloc(P, reinterpret_cast<double2**>(&P.d_spec), 3 * (size_t)fp::spec_capacity(P)),
+            "cudaMalloc spec");
     const size_t nparts = (size_t)std::max<long long>(fp::kMaxPartials, P.nrows + 64);
     FP_CUDA(dalloc(P, &P.d_partials, 4 * nparts), "cudaMalloc partials");
     FP_CUDA(dalloc(P, &P.d_red, 64), "cudaMalloc red");

@@ -68,9 +68,43 @@ template <typename T2>
 __device__ __forceinline__ T2 cmul(T2 a, T2 b) {
     return cmk<T2>(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
+
+// FP32 complex values as packed pairs: one f32x2 instruction does both parts
+// (each rounded as the scalar operation rounds).  The FP32 passes are bound by
+// instruction issue as much as by memory, and the packed form takes half the
+// issue slots at the same FP32 rate (measured: 120 lane operations per clock
+// and SM either way, 60 packed instructions).
+__device__ __forceinline__ unsigned long long f2_bits(float2 a) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
+    return r;
+}
+__device__ __forceinline__ float2 bits_f2(unsigned long long v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+template <>
+__device__ __forceinline__ float2 cadd<float2>(float2 a, float2 b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+    return bits_f2(r);
+}
+template <>
+__device__ __forceinline__ float2 csub<float2>(float2 a, float2 b) {
+    unsigned long long r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+    return bits_f2(r);
+}
 template <typename T2>
 __device__ __forceinline__ T2 cscale(T2 a, decltype(T2::x) s) {
     return cmk<T2>(a.x * s, a.y * s);
+}
+template <>
+__device__ __forceinline__ float2 cscale<float2>(float2 a, float s) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(make_float2(s, s))));
+    return bits_f2(r);
 }
 template <typename T2>
 __device__ __forceinline__ T2 cconj(T2 a) {
@@ -80,6 +114,17 @@ __device__ __forceinline__ T2 cconj(T2 a) {
 template <int SIGN, typename T2>
 __device__ __forceinline__ T2 cmul_si(T2 a) {
     return SIGN < 0 ? cmk<T2>(a.y, -a.x) : cmk<T2>(-a.y, a.x);
+}
+
+// a + sign*i*b and a - sign*i*b as two scalar additions: the rotated operand is
+// never formed (a packed addition would have to swap its halves first)
+template <int SIGN, typename T2>
+__device__ __forceinline__ T2 cadd_si(T2 a, T2 b) {
+    return SIGN < 0 ? cmk<T2>(a.x + b.y, a.y - b.x) : cmk<T2>(a.x - b.y, a.y + b.x);
+}
+template <int SIGN, typename T2>
+__device__ __forceinline__ T2 csub_si(T2 a, T2 b) {
+    return cadd_si<-SIGN>(a, b);
 }
 
 __device__ __forceinline__ double warp_sum(double v) {

@@ -33,9 +33,8 @@ cudaError_t run_xfwd(int n, const FastArgs& a, dim3 grid, int threads, size_t sm
 }
 
 template <typename T>
-cudaError_t run_xinv(int n, const FastArgs& a, int stage_bytes, dim3 grid, int threads, size_t smem,
-                     cudaStream_t s) {
-#define FP_CALL(N) Passes<T, N>::xinv(a, stage_bytes, grid, threads, smem, s)
+cudaError_t run_xinv(int n, const FastArgs& a, dim3 grid, int threads, size_t smem, cudaStream_t s) {
+#define FP_CALL(N) Passes<T, N>::xinv(a, grid, threads, smem, s)
     FP_EDGE_SWITCH(n, FP_CALL)
 #undef FP_CALL
     return cudaErrorInvalidValue;
@@ -99,8 +98,8 @@ namespace {
 template <typename T>
 struct FastPlan {
     fast::FastArgs a{};
-    int xthreads = 0, stage_bytes = 0, xgrid_f = 0, xgrid_i = 0, zstages = 2, zgrid = 0;
-    size_t xsmem = 0, xismem = 0, zsmem = 0;
+    int xthreads = 0, xgrid_f = 0, xgrid_i = 0, zstages = 2, zgrid = 0;
+    size_t xsmem = 0, zsmem = 0;
     dim3 ygrid;
     const CUtensorMap* smap = nullptr;
     const CUtensorMap* gmap = nullptr;
@@ -116,16 +115,17 @@ cudaError_t fast_plan(Problem& P, const ApplyArgs& aa, FastPlan<T>& pl) {
     a.nz = P.nz;
     a.nxh = P.nxh;
     a.rs = P.rs;
-    a.nh = P.nh;
+    a.nh = fast::spec_elems(P.nx, P.ny, P.nz);
     a.nrows = P.nrows;
     a.n = P.n;
-    a.plane = (long long)P.ny * P.rs;
-    a.tw32x = P.px.tw32;
-    a.tw32y = P.py.tw32;
-    a.tw32z = P.pz.tw32;
-    a.tw64x = P.px.tw64;
-    a.tw64y = P.py.tw64;
-    a.tw64z = P.pz.tw64;
+    a.ktl = fast::kt_log2(P.nx);
+    a.kts = P.nrows << a.ktl;
+    a.tw32x = P.px.fw32;
+    a.tw32y = P.py.fw32;
+    a.tw32z = P.pz.fw32;
+    a.tw64x = P.px.fw64;
+    a.tw64y = P.py.fw64;
+    a.tw64z = P.pz.fw64;
     a.spec = P.d_spec;
     a.green = sizeof(T) == 8 ? (const void*)P.d_green64 : (const void*)P.d_green32;
     a.support = P.d_support;
@@ -149,13 +149,8 @@ cudaError_t fast_plan(Problem& P, const ApplyArgs& aa, FastPlan<T>& pl) {
     a.ntiles = (P.nrows + rows - 1) / rows;
     pl.xthreads = ((3 * rows / 2 * fast::x_tpl(P.nx) + 31) / 32) * 32;
     pl.xsmem = (size_t)(3 * rows / 2) * fast::x_ld_rt<T>(P.nx) * sizeof(T2);
-    // inverse x: two stages, each the raw half-spectrum rows of a tile or,
-    // after stage A, its padded lines
-    const size_t raw = (size_t)3 * rows * P.rs * sizeof(T2);
-    pl.stage_bytes = (int)((std::max(raw, pl.xsmem) + 15) & ~size_t(15));
-    pl.xismem = 2 * (size_t)pl.stage_bytes;
     const int fwd_per_sm = fast::x_blocks_per_sm<T>(P.nx, false, pl.xthreads, pl.xsmem);
-    const int inv_per_sm = fast::x_blocks_per_sm<T>(P.nx, true, pl.xthreads, pl.xismem);
+    const int inv_per_sm = fast::x_blocks_per_sm<T>(P.nx, true, pl.xthreads, pl.xsmem);
     pl.xgrid_f = (int)std::min<long long>(a.ntiles, (long long)fwd_per_sm * P.sm_count);
     pl.xgrid_i = (int)std::min<long long>(a.ntiles, (long long)inv_per_sm * P.sm_count);
     pl.xgrid_i = std::min(pl.xgrid_i, kMaxPartials);
@@ -199,7 +194,7 @@ cudaError_t fast_run(const Problem& P, const FastPlan<T>& pl, const fast::FastAr
         e = fast::run_z<T>(P.nz, pl.zstages, *pl.smap, *pl.gmap, a, dim3(zgrid, G), pl.zsmem, st);
     if (e != cudaSuccess) return e;
     if ((e = fast::run_y<T>(P.ny, +1, a, yg, st)) != cudaSuccess) return e;
-    return fast::run_xinv<T>(P.nx, a, pl.stage_bytes, dim3(pl.xgrid_i, G), pl.xthreads, pl.xismem, st);
+    return fast::run_xinv<T>(P.nx, a, dim3(pl.xgrid_i, G), pl.xthreads, pl.xsmem, st);
 }
 
 template <typename T>
@@ -221,7 +216,7 @@ cudaError_t member_impl(Problem& P, const ApplyArgs& aa, fast::FastArgs* args, C
     *args = pl.a;
     maps[0] = *pl.smap;
     maps[1] = *pl.gmap;
-    const long long g[kGroupGeometry] = {P.nx, P.ny, P.nz, pl.a.rows, pl.xthreads, pl.stage_bytes,
+    const long long g[kGroupGeometry] = {P.nx, P.ny, P.nz, pl.a.rows, pl.xthreads, (long long)pl.xsmem,
                                          pl.xgrid_f, pl.xgrid_i, pl.zstages, (long long)pl.zsmem,
                                          pl.zgrid, P.rs};
     for (int i = 0; i < kGroupGeometry; ++i) geometry[i] = g[i];

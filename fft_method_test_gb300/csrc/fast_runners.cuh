@@ -22,12 +22,11 @@ cudaError_t Passes<T, N>::xfwd(const FastArgs& a, dim3 grid, int threads, size_t
 }
 
 template <typename T, int N>
-cudaError_t Passes<T, N>::xinv(const FastArgs& a, int stage_bytes, dim3 grid, int threads, size_t smem,
-                               cudaStream_t s) {
+cudaError_t Passes<T, N>::xinv(const FastArgs& a, dim3 grid, int threads, size_t smem, cudaStream_t s) {
     if (a.group)
-        FP_RUN((k_fx_inv<T, N, true>), grid, threads, smem, s, a, stage_bytes);
+        FP_RUN((k_fx_inv<T, N, true>), grid, threads, smem, s, a);
     else
-        FP_RUN((k_fx_inv<T, N, false>), grid, threads, smem, s, a, stage_bytes);
+        FP_RUN((k_fx_inv<T, N, false>), grid, threads, smem, s, a);
     return cudaGetLastError();
 }
 

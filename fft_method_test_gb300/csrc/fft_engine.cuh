@@ -110,14 +110,17 @@ __device__ __forceinline__ void dft2(T2& a, T2& b) {
     b = csub(t, b);
 }
 
-template <int S, typename T2>
+// With ROT2 the third input enters multiplied by S*i (the twiddle of a larger
+// transform, taken by the additions instead of a rotation of its own).
+template <int S, bool ROT2 = false, typename T2>
 __device__ __forceinline__ void dft4(T2& x0, T2& x1, T2& x2, T2& x3) {
-    const T2 s02 = cadd(x0, x2), d02 = csub(x0, x2);
-    const T2 s13 = cadd(x1, x3), d13 = cmul_si<S>(csub(x1, x3));
+    const T2 s02 = ROT2 ? cadd_si<S>(x0, x2) : cadd(x0, x2);
+    const T2 d02 = ROT2 ? csub_si<S>(x0, x2) : csub(x0, x2);
+    const T2 s13 = cadd(x1, x3), d13 = csub(x1, x3);
     x0 = cadd(s02, s13);
     x2 = csub(s02, s13);
-    x1 = cadd(d02, d13);
-    x3 = csub(d02, d13);
+    x1 = cadd_si<S>(d02, d13);
+    x3 = csub_si<S>(d02, d13);
 }
 
 template <int S, typename T2>
@@ -127,10 +130,10 @@ __device__ __forceinline__ void dft3(T2& x0, T2& x1, T2& x2) {
     const T2 t1 = cadd(x1, x2);
     const T2 t2 = cmk<T2>(x0.x - (T)0.5 * t1.x, x0.y - (T)0.5 * t1.y);
     const T2 d = csub(x1, x2);
-    const T2 t3 = cmul_si<S>(cmk<T2>(kS3 * d.x, kS3 * d.y));
+    const T2 t3 = cmk<T2>(kS3 * d.x, kS3 * d.y);
     x0 = cadd(x0, t1);
-    x1 = cadd(t2, t3);
-    x2 = csub(t2, t3);
+    x1 = cadd_si<S>(t2, t3);
+    x2 = csub_si<S>(t2, t3);
 }
 
 template <int S, typename T2>
@@ -144,13 +147,13 @@ __device__ __forceinline__ void dft5(T2& x0, T2& x1, T2& x2, T2& x3, T2& x4) {
     const T2 p23 = cadd(x2, x3), m23 = csub(x2, x3);
     const T2 a1 = cmk<T2>(x0.x + c1 * p14.x + c2 * p23.x, x0.y + c1 * p14.y + c2 * p23.y);
     const T2 a2 = cmk<T2>(x0.x + c2 * p14.x + c1 * p23.x, x0.y + c2 * p14.y + c1 * p23.y);
-    const T2 b1 = cmul_si<S>(cmk<T2>(s1 * m14.x + s2 * m23.x, s1 * m14.y + s2 * m23.y));
-    const T2 b2 = cmul_si<S>(cmk<T2>(s2 * m14.x - s1 * m23.x, s2 * m14.y - s1 * m23.y));
+    const T2 b1 = cmk<T2>(s1 * m14.x + s2 * m23.x, s1 * m14.y + s2 * m23.y);
+    const T2 b2 = cmk<T2>(s2 * m14.x - s1 * m23.x, s2 * m14.y - s1 * m23.y);
     x0 = cadd(x0, cadd(p14, p23));
-    x1 = cadd(a1, b1);
-    x4 = csub(a1, b1);
-    x2 = cadd(a2, b2);
-    x3 = csub(a2, b2);
+    x1 = cadd_si<S>(a1, b1);
+    x4 = csub_si<S>(a1, b1);
+    x2 = cadd_si<S>(a2, b2);
+    x3 = csub_si<S>(a2, b2);
 }
 
 // multiply by exp(S * i * pi / 4) and exp(S * 3 i pi / 4)
@@ -158,13 +161,13 @@ template <int S, typename T2>
 __device__ __forceinline__ T2 mul_w8_1(T2 a) {
     using T = decltype(T2::x);
     const T c = (T)0.70710678118654752440;
-    return S < 0 ? cmk<T2>(c * (a.x + a.y), c * (a.y - a.x)) : cmk<T2>(c * (a.x - a.y), c * (a.y + a.x));
+    return cscale(cadd_si<S>(a, a), c);  // (1 + S i) a / sqrt(2)
 }
 template <int S, typename T2>
 __device__ __forceinline__ T2 mul_w8_3(T2 a) {
     using T = decltype(T2::x);
     const T c = (T)0.70710678118654752440;
-    return S < 0 ? cmk<T2>(c * (a.y - a.x), -c * (a.x + a.y)) : cmk<T2>(-c * (a.x + a.y), c * (a.x - a.y));
+    return cscale(csub_si<S>(a, a), -c);  // (-1 + S i) a / sqrt(2)
 }
 
 // DFT8 as 2 x 4: y[2q] = DFT4(x_r + x_{r+4})[q], y[2q+1] = DFT4((x_r - x_{r+4}) W8^r)[q].
@@ -174,10 +177,9 @@ __device__ __forceinline__ void dft8(T2 (&v)[8]) {
 #pragma unroll
     for (int r = 0; r < 4; ++r) dft2<S>(v[r], v[r + 4]);
     v[5] = mul_w8_1<S>(v[5]);
-    v[6] = cmul_si<S>(v[6]);
     v[7] = mul_w8_3<S>(v[7]);
     dft4<S>(v[0], v[1], v[2], v[3]);
-    dft4<S>(v[4], v[5], v[6], v[7]);
+    dft4<S, true>(v[4], v[5], v[6], v[7]);  // v[6] times S*i
 }
 
 template <int S, typename T2>
@@ -193,21 +195,21 @@ __device__ __forceinline__ void dft16(T2 (&v)[16]) {
     using T = decltype(T2::x);
     const T c8 = (T)0.92387953251128675613;   // cos(pi/8)
     const T s8 = (T)0.38268343236508977173;   // sin(pi/8)
-    const T h = (T)0.70710678118654752440;
 #pragma unroll
     for (int b = 0; b < 4; ++b) dft4<S>(v[b], v[4 + b], v[8 + b], v[12 + b]);
     // t_b[c] lives in v[4c + b]; multiply by W16^(b*c)
     v[5] = mul_const<S>(v[5], c8, s8);     // W^1
-    v[6] = mul_const<S>(v[6], h, h);       // W^2
+    v[6] = mul_w8_1<S>(v[6]);       // W^2
     v[7] = mul_const<S>(v[7], s8, c8);     // W^3
-    v[9] = mul_const<S>(v[9], h, h);       // W^2
-    v[10] = cmul_si<S>(v[10]);             // W^4
-    v[11] = mul_const<S>(v[11], -h, h);    // W^6
+    v[9] = mul_w8_1<S>(v[9]);       // W^2
+    v[11] = mul_w8_3<S>(v[11]);    // W^6
     v[13] = mul_const<S>(v[13], s8, c8);   // W^3
-    v[14] = mul_const<S>(v[14], -h, h);    // W^6
+    v[14] = mul_w8_3<S>(v[14]);    // W^6
     v[15] = mul_const<S>(v[15], -c8, -s8); // W^9
-#pragma unroll
-    for (int c = 0; c < 4; ++c) dft4<S>(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+    dft4<S>(v[0], v[1], v[2], v[3]);
+    dft4<S>(v[4], v[5], v[6], v[7]);
+    dft4<S, true>(v[8], v[9], v[10], v[11]);  // v[10] times W^4 = S*i
+    dft4<S>(v[12], v[13], v[14], v[15]);
 }
 
 // register holding output k of dft_r<R>

@@ -26,9 +26,7 @@
 //              tiles of the next (kx, ky) tile load while the current one is
 //              transformed)
 //   k_fx_inv   C2R x lines, gather to the support, 1/N scale, per-CTA partial
-//              sums (component sums and the dot with a given vector);
-//              persistent CTAs, the next tile's half-spectrum rows arriving
-//              by cp.async while the current tile is transformed
+//              sums (component sums and the dot with a given vector)
 //
 // Shared-memory line strides are chosen so that the half-warp (FP32) or
 // quarter-warp (FP64) of every exchange touches distinct banks.
@@ -134,12 +132,16 @@ __device__ __forceinline__ void dft_pfa(T2 (&v)[P * Q]) {
     for (int k = 0; k < R; ++k) v[k] = a[k % P][k % Q];
 }
 
-// twiddle W_N^(S e) from the table tw[j] = exp(-2 pi i j / N), 0 <= e < N
-template <int S, typename T2>
-__device__ __forceinline__ T2 twiddle(const T2* __restrict__ tw, int e) {
-    T2 w = __ldg(tw + e);
-    if (S > 0) w.y = -w.y;
-    return w;
+// Twiddle W_N^(S a k) of output k of owner a between the two stages, N = RA*RB.
+// The tables hold them in the order the threads read them, [k][a], so that the
+// owners of one warp instruction read neighbouring entries: indexing one table
+// of N roots by a*k touches up to RB cache lines per load, and the L1 data pipe
+// is the busiest unit of these passes (65-87 % of its peak under ncu).  Measured
+// at 256^3 FP32: 431.6 -> 425.0 us per apply.
+// The forward table [R1][R2] is followed by the inverse one [R2][R1], conjugated.
+template <int RA, int RB, int S, typename T2>
+__device__ __forceinline__ T2 twiddle(const T2* __restrict__ tw, int k, int a) {
+    return __ldg(tw + (S > 0 ? RA * RB : 0) + k * RB + a);
 }
 
 // ---- line strides ------------------------------------------------------------
@@ -187,6 +189,11 @@ struct GroupBarrier {
     }
 };
 
+// one warp: the threads of a line in the x passes (TPL divides 32)
+struct WarpBarrier {
+    __device__ __forceinline__ void operator()() const { __syncwarp(); }
+};
+
 template <class B>
 __device__ __forceinline__ B make_group_barrier(int id, int count);
 template <>
@@ -224,7 +231,7 @@ __device__ __forceinline__ void stage_a(T2* line, int t, bool active, const T2* 
 #pragma unroll
             for (int k = 0; k < RA; ++k) {
                 T2 y = v[j][k];
-                if (k > 0) y = cmul(y, twiddle<S>(tw, a * k));  // a * k < N
+                if (k > 0) y = cmul(y, twiddle<RA, RB, S>(tw, k, a));
                 line[k * (RB + 1) + a] = y;
             }
         }
@@ -258,12 +265,60 @@ __device__ __forceinline__ void stage_b(const T2* line, int t, bool active, Stor
     }
 }
 
+// Stage A with its inputs already in registers (z[j][i] = x[RB*i + t + TPL*j]);
+// the line is free to be written.
+template <int RA, int RB, int S, int TPL, typename T2>
+__device__ __forceinline__ void stage_a_regs(T2* line, int t, bool active, const T2* __restrict__ tw,
+                                             T2 (&z)[RB / TPL][RA]) {
+    if (!active) return;
+#pragma unroll
+    for (int j = 0; j < RB / TPL; ++j) {
+        const int a = t + TPL * j;
+        dft_nat<RA, S>(z[j]);
+#pragma unroll
+        for (int k = 0; k < RA; ++k) {
+            T2 y = z[j][k];
+            if (k > 0) y = cmul(y, twiddle<RA, RB, S>(tw, k, a));
+            line[k * (RB + 1) + a] = y;
+        }
+    }
+}
+
+// Stage B leaving its outputs in registers: z[j][m] = X[t + TPL*j + RA*m].
+template <int RA, int RB, int S, int TPL, typename T2>
+__device__ __forceinline__ void stage_b_regs(const T2* line, int t, bool active, T2 (&z)[RA / TPL][RB]) {
+#pragma unroll
+    for (int j = 0; j < RA / TPL; ++j)
+#pragma unroll
+        for (int a = 0; a < RB; ++a) z[j][a] = active ? line[(t + TPL * j) * (RB + 1) + a] : T2{};
+#pragma unroll
+    for (int j = 0; j < RA / TPL; ++j) dft_nat<RB, S>(z[j]);
+}
+
+// ---- spectral layout -----------------------------------------------------------
+
+// The spectral field between the specialised passes is blocked over kx in
+// tiles of kt = 2^ktl columns: element (comp, kx, ky, kz) sits at
+//   comp * nh + (kx / kt) * kts + (kz * ny + ky) * kt + kx % kt,  kts = kt * ny * nz,
+// so a y line of a tile is one contiguous block and the lines of a z tile are
+// ny * kt elements apart.  kt is the number of threads of an x line: a load or
+// store of the x passes covers one tile row whole (with a narrower tile it
+// touched a cache line per 32 bytes).  Measured per mixed apply, [kz][ky][kx]
+// against this layout: 64^3 32.7 -> 30.4 us, 128^3 80.0 -> 74.9, 160^3 152.5 ->
+// 140.2, 256^3 425 -> 431 (its y passes 72 -> 63 us, its x passes as much slower).
+template <int N>
+__host__ __device__ constexpr int kx_tile() {
+    return Split<N>::TPL < 4 ? 4 : Split<N>::TPL;
+}
+
 // ---- kernel arguments ----------------------------------------------------------
 
 struct FastArgs {
     int nx, ny, nz, nxh;
-    long long rs, nh, nrows, n, plane;
-    const float2* tw32x;
+    long long rs, nh, nrows, n;
+    int ktl;        // log2 of the kx tile width
+    long long kts;  // elements of one kx tile of a component
+    const float2* tw32x;  // stage twiddles of the specialised edges (AxisPlan::fw32)
     const float2* tw32y;
     const float2* tw32z;
     const double2* tw64x;
@@ -314,18 +369,84 @@ __host__ __device__ constexpr int x_threads(int rows) {
     return ((3 * rows / 2 * Split<N>::TPL + 31) / 32) * 32;
 }
 
-// ---- cp.async (global -> shared, completion by group) ---------------------------
+// ---- two real lines in one complex line --------------------------------------
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
-                     static_cast<uint32_t>(__cvta_generic_to_shared(smem))),
-                 "l"(gmem)
-                 : "memory");
+// A thread t of a line's TPL threads holds Z[k] for k = t + TPL*j + R1*m in
+// z[j][m] (j < R1/TPL, m < R2): the owners of the forward transform's stage B
+// and of the inverse transform's stage A.  Z[N - k] then sits in register
+// [J-1-j][R2-1-m] of thread (TPL - t) % TPL, except for t = 0, whose mirror
+// images are its own registers: the two Hermitian halves meet through warp
+// shuffles, without shared memory.
+
+// the value of `v` in the mirror thread
+template <int TPL>
+__device__ __forceinline__ float2 shfl_mirror(float2 v, int t) {
+    const int src = (TPL - t) & (TPL - 1);
+    return make_float2(__shfl_sync(0xffffffffu, v.x, src, TPL), __shfl_sync(0xffffffffu, v.y, src, TPL));
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int PENDING>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
+template <int TPL>
+__device__ __forceinline__ double2 shfl_mirror(double2 v, int t) {
+    const int src = (TPL - t) & (TPL - 1);
+    return make_double2(__shfl_sync(0xffffffffu, v.x, src, TPL), __shfl_sync(0xffffffffu, v.y, src, TPL));
+}
+
+template <class T2>
+__device__ __forceinline__ T2 pick(bool c, T2 a, T2 b) {
+    return cmk<T2>(c ? a.x : b.x, c ? a.y : b.y);
+}
+
+// Spectra of the two real lines of a forward line, each times two:
+// store(k, 2 A[k], 2 B[k]) for this thread's k <= N/2.
+template <int R1, int R2, int TPL, typename T2, class Store>
+__device__ __forceinline__ void separate_lines(const T2 (&z)[R1 / TPL][R2], int t, Store& store) {
+    static_assert(R2 % 2 == 0, "the half spectrum is the lower half of the outputs");
+    constexpr int J = R1 / TPL;
+#pragma unroll
+    for (int m = 0; m < R2 / 2; ++m)
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            const T2 own = j > 0 ? z[j > 0 ? J - j : 0][R2 - 1 - m] : z[0][(R2 - m) % R2];
+            const T2 zn = pick(t == 0, own, shfl_mirror<TPL>(z[J - 1 - j][R2 - 1 - m], t));
+            const T2 zk = z[j][m];
+            store(t + TPL * j + R1 * m, cmk<T2>(zk.x + zn.x, zk.y - zn.y), cmk<T2>(zk.y + zn.y, zn.x - zk.x));
+        }
+    if (t == 0) {  // k = N/2 is its own mirror image
+        using T = decltype(T2::x);
+        const T2 zk = z[0][R2 / 2];
+        store(R1 * R2 / 2, cmk<T2>(zk.x + zk.x, (T)0), cmk<T2>(zk.y + zk.y, (T)0));
+    }
+}
+
+// The inverse: z[j][m] of Z = A + iB from the half spectra, load(k, A, B) for
+// this thread's k <= N/2 (DC and Nyquist are real).
+template <int R1, int R2, int TPL, typename T2, class Load>
+__device__ __forceinline__ void join_lines(T2 (&z)[R1 / TPL][R2], int t, Load& load) {
+    using T = decltype(T2::x);
+    constexpr int J = R1 / TPL;
+    constexpr int H = R2 / 2;
+    T2 a[J][H], b[J][H], an{}, bn{};
+#pragma unroll
+    for (int m = 0; m < H; ++m)
+#pragma unroll
+        for (int j = 0; j < J; ++j) load(t + TPL * j + R1 * m, a[j][m], b[j][m]);
+    if (t == 0) load(R1 * H, an, bn);
+    if (t == 0) a[0][0].y = b[0][0].y = (T)0;
+    T2 w[J][H];  // Z[N - k]
+#pragma unroll
+    for (int m = 0; m < H; ++m)
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            z[j][m] = cmk<T2>(a[j][m].x - b[j][m].y, a[j][m].y + b[j][m].x);
+            w[j][m] = cmk<T2>(a[j][m].x + b[j][m].y, b[j][m].x - a[j][m].y);
+        }
+    const T2 nyq = cmk<T2>(an.x, bn.x);
+#pragma unroll
+    for (int m = 0; m < H; ++m)
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            const T2 own = j + 1 < J ? w[j + 1 < J ? j + 1 : 0][m] : (m + 1 < H ? w[0][m + 1 < H ? m + 1 : 0] : nyq);
+            z[J - 1 - j][R2 - 1 - m] = pick(t == 0, own, shfl_mirror<TPL>(w[j][m], t));
+        }
 }
 
 // ---- P1: scatter + R2C x -------------------------------------------------------
@@ -333,15 +454,13 @@ __device__ __forceinline__ void cp_async_wait() {
 // complex lines per tile of the x passes at most (3 * rows / 2, rows <= 32)
 constexpr int kMaxXLines = 48;
 
-// two neighbouring complex values to 16-byte aligned global memory
-__device__ __forceinline__ void store_pair(float2* p, float2 a, float2 b) {
-    *reinterpret_cast<float4*>(p) = make_float4(a.x, a.y, b.x, b.y);
-}
-__device__ __forceinline__ void store_pair(double2* p, double2 a, double2 b) {
-    p[0] = a;
-    p[1] = b;
-}
-
+// One line's threads share a warp, so the stages of a line exchange through
+// shared memory with warp barriers, and the half spectra leave the registers
+// for HBM directly (a store covers TPL neighbouring kx).  The two spectra are
+// stored times two; the inverse pass takes the factor back with its 1/N.
+// Against separating the spectra through shared memory: 49 -> 35 M warp
+// instructions, 80.3 -> 69.7 us at 256^3 FP32 under ncu; L1 and latency bound
+// it (DRAM at 33 %, 22 warps per SM).
 template <typename T, int N, bool GROUP>
 __global__ void __launch_bounds__(384) k_fx_fwd(const __grid_constant__ FastArgs a0) {
     // a group member's arguments are copied out of the table once: read
@@ -351,10 +470,10 @@ __global__ void __launch_bounds__(384) k_fx_fwd(const __grid_constant__ FastArgs
     if (a.skip && *a.skip) return;
     using T2 = c_t<T>;
     constexpr int R1 = Split<N>::R1, R2 = Split<N>::R2, TPL = Split<N>::TPL;
+    constexpr int KT = kx_tile<N>();
+    static_assert(32 % TPL == 0, "the threads of a line share a warp");
     constexpr int LD = x_ld<N, T>();
-    constexpr int NH = N / 2 + 1;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    __shared__ long long dst_a[kMaxXLines], dst_b[kMaxXLines];
     T2* lines = reinterpret_cast<T2*>(smem_raw);
     const int RB = a.rows;
     const int nq = 3 * RB / 2;
@@ -367,6 +486,8 @@ __global__ void __launch_bounds__(384) k_fx_fwd(const __grid_constant__ FastArgs
     const T mean[3] = {a.src_sum ? (T)(a.src_sum[0] * a.inv_nb) : (T)0,
                        a.src_sum ? (T)(a.src_sum[1] * a.inv_nb) : (T)0,
                        a.src_sum ? (T)(a.src_sum[2] * a.inv_nb) : (T)0};
+    const int La = 2 * q, rla = La / 3, ca = La - 3 * rla;
+    const int Lb = La + 1, rlb = Lb / 3, cb = Lb - 3 * rlb;
     for (long long tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x) {
         const long long r0 = tile * RB;
         const int rows = (int)min((long long)RB, a.nrows - r0);
@@ -396,69 +517,50 @@ __global__ void __launch_bounds__(384) k_fx_fwd(const __grid_constant__ FastArgs
         }
         __syncthreads();
         // 3) forward FFT of every complex line (stage A reads the natural line,
-        //    stage B leaves X in registers, written back in natural order)
+        //    stage B leaves X in registers), half spectra to HBM
         const bool act = q < nqa;
         T2* my = lines + (act ? q : 0) * LD;
+        T2 z[R1 / TPL][R2];
         {
             auto ld_nat = [&](int pos) { return my[pos]; };
-            stage_a<R1, R2, -1, TPL, true>(my, t, act, tw, ld_nat);
-            __syncthreads();
-            auto st_nat = [&](int pos, T2 v) { my[pos] = v; };
-            stage_b<R1, R2, -1, TPL, true>(my, t, act, st_nat);
+            stage_a<R1, R2, -1, TPL, true>(my, t, act, tw, ld_nat, WarpBarrier{});
+            __syncwarp();
+            stage_b_regs<R1, R2, -1, TPL>(my, t, act, z);
         }
-        __syncthreads();
-        // 4) separate the two real spectra of each complex line, store the half
-        //    spectra, two neighbouring kx per thread (one 16-byte store for
-        //    FP32; rs is a multiple of 4, so every even kx is 16-byte aligned;
-        //    kx = N/2 + 1 lands in the row padding)
-        if (tid < nqa) {
-            const int La = 2 * tid, rla = La / 3, ca = La - 3 * rla;
-            dst_a[tid] = ca * a.nh + (r0 + rla) * a.rs;
-            const int Lb = La + 1, rlb = Lb / 3, cb = Lb - 3 * rlb;
-            dst_b[tid] = Lb < nreal ? cb * a.nh + (r0 + rlb) * a.rs : -1;
+        {
+            T2* pa = spec + ca * a.nh + (r0 + rla) * KT;
+            T2* pb = spec + cb * a.nh + (r0 + rlb) * KT;
+            const bool hasb = act && Lb < nreal;
+            auto st = [&](int k, T2 A, T2 B) {
+                const long long o = (k / KT) * a.kts + k % KT;
+                if (act) pa[o] = A;
+                if (hasb) pb[o] = B;
+            };
+            separate_lines<R1, R2, TPL>(z, t, st);
         }
-        __syncthreads();
-        constexpr int NP = (NH + 1) / 2;
-        for (int it = tid; it < nqa * NP; it += nthr) {
-            const int qq = it / NP;
-            const int k = 2 * (it - qq * NP);
-            const T2* ln = lines + qq * LD;
-            T2 A[2], B[2];
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int kk = k + e;
-                const T2 zk = ln[kk];
-                const T2 zn = ln[kk == 0 ? 0 : N - kk];
-                const T h = (T)0.5;
-                A[e] = cmk<T2>(h * (zk.x + zn.x), h * (zk.y - zn.y));
-                B[e] = cmk<T2>(h * (zk.y + zn.y), h * (zn.x - zk.x));
-            }
-            store_pair(spec + dst_a[qq] + k, A[0], A[1]);
-            if (dst_b[qq] >= 0) store_pair(spec + dst_b[qq] + k, B[0], B[1]);
-        }
-        __syncthreads();
+        __syncthreads();  // the lines are zeroed by the next tile
     }
 }
 
 // ---- P5: C2R x + gather + partial sums -------------------------------------------
 
-// Persistent CTAs walk tiles of `rows` grid rows.  The three component blocks
-// of a tile are contiguous rows of the half spectrum; cp.async brings the next
-// tile's rows into the other of two shared-memory stages while the current
-// tile is transformed.  Stage A of the inverse transform builds the complex
-// lines Z = A + iB of two real lines straight from the raw Hermitian half
-// spectra ([comp][row][rs], as copied); after a barrier the padded lines
-// overwrite the same stage.  stage_bytes covers the larger of the two layouts.
+// Persistent CTAs walk tiles of `rows` grid rows.  Bound by L1 and the latency
+// of its loads (DRAM at 37 %).  Each thread reads its part
+// of the two half spectra of a line straight from HBM (TPL neighbouring kx per
+// load), so shared memory holds the lines of the exchange only and several
+// CTAs per SM cover the latency of each other's loads.  Against the former
+// form (raw rows staged by cp.async, Hermitian halves read from shared memory):
+// 60 -> 33 M warp instructions, 82.8 -> 70.4 us at 256^3 FP32 under ncu.
 template <typename T, int N, bool GROUP>
-__global__ void __launch_bounds__(384) k_fx_inv(const __grid_constant__ FastArgs a0, int stage_bytes) {
+__global__ void __launch_bounds__(384) k_fx_inv(const __grid_constant__ FastArgs a0) {
     const FastArgs ag = GROUP ? a0.group[blockIdx.y] : FastArgs{};
     const FastArgs& a = GROUP ? ag : a0;
     if (a.skip && *a.skip) return;
     using T2 = c_t<T>;
     constexpr int R1 = Split<N>::R1, R2 = Split<N>::R2, TPL = Split<N>::TPL;
+    constexpr int KT = kx_tile<N>();
+    static_assert(32 % TPL == 0, "the threads of a line share a warp");
     constexpr int LD = x_ld<N, T>();
-    constexpr int NH = N / 2 + 1;
-    constexpr int SPC = 16 / sizeof(T2);  // elements per 16-byte copy
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ double red[4 * 32];
     const int RB = a.rows;
@@ -468,38 +570,14 @@ __global__ void __launch_bounds__(384) k_fx_inv(const __grid_constant__ FastArgs
     const int t = tid - q * TPL;
     const T2* tw = tw_of<T>(a, 0);
     const T2* spec = reinterpret_cast<const T2*>(a.spec);
-    const T scale = (T)a.scale;
-    const long long rs = a.rs;
+    T2* lines = reinterpret_cast<T2*>(smem_raw);
+    const T scale = (T)(0.5 * a.scale);  // the forward pass stores twice the spectra
     T acc[4] = {(T)0, (T)0, (T)0, (T)0};
+    // complex line q carries real lines 2q (A) and 2q + 1 (B)
+    const int La = 2 * q, rla = La / 3, ca = La - 3 * rla;
+    const int Lb = La + 1, rlb = Lb / 3, cb = Lb - 3 * rlb;
 
-    auto issue = [&](long long tile, int st) {
-        T2* raw = reinterpret_cast<T2*>(smem_raw + st * (size_t)stage_bytes);
-        const long long r0 = tile * RB;
-        const int rows = (int)min((long long)RB, a.nrows - r0);
-        const int per_comp = (int)(rows * rs / SPC);  // rs is a multiple of 4: whole copies
-        for (int i = tid; i < 3 * per_comp; i += nthr) {
-            const int cc = i / per_comp;
-            const int j = i - cc * per_comp;
-            cp_async16(raw + (size_t)cc * RB * rs + (size_t)j * SPC,
-                       spec + cc * a.nh + r0 * rs + (long long)j * SPC);
-        }
-        cp_async_commit();
-    };
-
-    long long tile = blockIdx.x;
-    if (tile < a.ntiles) issue(tile, 0);
-    for (int it = 0; tile < a.ntiles; tile += gridDim.x, ++it) {
-        const int st = it & 1;
-        const long long next = tile + gridDim.x;
-        if (next < a.ntiles) {
-            issue(next, st ^ 1);
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
-        }
-        __syncthreads();
-        const T2* raw = reinterpret_cast<const T2*>(smem_raw + st * (size_t)stage_bytes);
-        T2* lines = reinterpret_cast<T2*>(smem_raw + st * (size_t)stage_bytes);
+    for (long long tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x) {
         const long long r0 = tile * RB;
         const int rows = (int)min((long long)RB, a.nrows - r0);
         const int nreal = 3 * rows;
@@ -507,33 +585,22 @@ __global__ void __launch_bounds__(384) k_fx_inv(const __grid_constant__ FastArgs
         const bool act = q < nqa;
         T2* my = lines + (act ? q : 0) * LD;
         {
-            // complex line q carries real lines 2q (A) and 2q + 1 (B)
-            const int La = 2 * q, rla = La / 3, ca = La - 3 * rla;
-            const int Lb = La + 1, rlb = Lb / 3, cb = Lb - 3 * rlb;
-            const T2* ra = raw + ((size_t)ca * RB + rla) * rs;
-            const T2* rb = raw + ((size_t)cb * RB + rlb) * rs;
-            const bool hasb = Lb < nreal;
-            auto ld_herm = [&](int k) {
-                const bool lo = k < NH;
-                const int kk = lo ? k : N - k;
-                T2 A = ra[kk];
-                T2 B = hasb ? rb[kk] : T2{};
-                if (kk == 0 || 2 * kk == N) {  // DC and Nyquist are real
-                    A.y = (T)0;
-                    B.y = (T)0;
-                }
-                if (!lo) {  // Z[k] = conj(A[N-k]) + i conj(B[N-k])
-                    A.y = -A.y;
-                    B.y = -B.y;
-                }
-                return cmk<T2>(A.x - B.y, A.y + B.x);
+            const T2* pa = spec + ca * a.nh + (r0 + rla) * KT;
+            const T2* pb = spec + cb * a.nh + (r0 + rlb) * KT;
+            const bool hasb = act && Lb < nreal;
+            auto ld = [&](int k, T2& A, T2& B) {
+                const long long o = (k / KT) * a.kts + k % KT;
+                A = act ? pa[o] : T2{};
+                B = hasb ? pb[o] : T2{};
             };
-            stage_a<R2, R1, +1, TPL, true>(my, t, act, tw, ld_herm);
+            T2 z[R1 / TPL][R2];
+            join_lines<R1, R2, TPL>(z, t, ld);
+            stage_a_regs<R2, R1, +1, TPL>(my, t, act, tw, z);
         }
-        __syncthreads();
+        __syncwarp();
         {
             auto st_nat = [&](int pos, T2 v) { my[pos] = v; };
-            stage_b<R2, R1, +1, TPL, true>(my, t, act, st_nat);
+            stage_b<R2, R1, +1, TPL, true>(my, t, act, st_nat, WarpBarrier{});
         }
         __syncthreads();
         // gather to the support with the 1/N scale, partial sums
@@ -556,7 +623,7 @@ __global__ void __launch_bounds__(384) k_fx_inv(const __grid_constant__ FastArgs
                 }
             }
         }
-        __syncthreads();  // this stage is refilled by the issue of iteration it + 1
+        __syncthreads();  // the lines are rewritten by the next tile
     }
     double accd[4] = {(double)acc[0], (double)acc[1], (double)acc[2], (double)acc[3]};
     double out[4];
@@ -586,9 +653,10 @@ __global__ void __launch_bounds__(TX * Split<N>::TPL) k_fcol_y(const __grid_cons
     const int k0 = blockIdx.x * TX;
     const bool act = k0 + c < a.nxh;
     const T2* tw = tw_of<T>(a, 1);
-    T2* base = reinterpret_cast<T2*>(a.spec) + comp * a.nh + (long long)blockIdx.y * N * a.rs +
-               k0 + (act ? c : 0);
-    const long long es = a.rs;
+    const int kx = k0 + (act ? c : 0);
+    T2* base = reinterpret_cast<T2*>(a.spec) + comp * a.nh + (kx >> a.ktl) * a.kts +
+               (((long long)blockIdx.y * N) << a.ktl) + (kx & ((1 << a.ktl) - 1));
+    const int es = 1 << a.ktl;
     T2* my = lines + c * LD;
     auto ld_g = [&](int pos) { return base[pos * es]; };
     auto st_g = [&](int pos, T2 v) { base[pos * es] = v; };
@@ -683,7 +751,8 @@ __global__ void __launch_bounds__(3 * TX * Split<N>::TPL, STAGES == 1 ? 3 : 1)
         const int ky = (int)(tile / ntx);
         mbar_arrive_expect_tx(&bars[st], TILE_BYTES);
         for (int cc = 0; cc < 3; ++cc)
-            tma_load_4d(base + (size_t)cc * CS * sizeof(T2), smap, 2 * k0, ky, 0, cc, &bars[st]);
+            tma_load_4d(base + (size_t)cc * CS * sizeof(T2), smap, 2 * ((ky << a.ktl) + (k0 & ((1 << a.ktl) - 1))), 0,
+                        k0 >> a.ktl, cc, &bars[st]);
         for (int gc = 0; gc < 6; ++gc)
             tma_load_4d(base + GOFF + (size_t)gc * N * TX * sizeof(T), gmap, k0, ky, 0, gc, &bars[st]);
     };
@@ -744,8 +813,9 @@ __global__ void __launch_bounds__(3 * TX * Split<N>::TPL, STAGES == 1 ? 3 : 1)
         }
         gbar();
         {
-            T2* base = reinterpret_cast<T2*>(a.spec) + comp * a.nh + ky * a.rs + k0 + (act ? c : 0);
-            const long long es = a.plane;
+            T2* base = reinterpret_cast<T2*>(a.spec) + comp * a.nh + (k0 >> a.ktl) * a.kts + (ky << a.ktl) +
+                       ((k0 + c) & ((1 << a.ktl) - 1));
+            const int es = a.ny << a.ktl;
             auto st_g = [&](int pos, T2 v) { base[pos * es] = v; };
             stage_b<R2, R1, +1, TPL, false>(my, t, act, st_g);
         }
@@ -814,8 +884,8 @@ __global__ void __launch_bounds__(3 * TX * Split<N>::TPL, sizeof(T) == 4 ? 2 : 1
         unsigned char* sb = spec0 + st * SPEC;
         mbar_arrive_expect_tx(&bars[st], SPEC_BYTES + (m == 0 ? GREEN_BYTES : 0u));
         for (int cc = 0; cc < 3; ++cc)
-            tma_load_4d(sb + (size_t)cc * CS * sizeof(T2), &a0.group_maps[2 * m], 2 * k0, ky, 0, cc,
-                        &bars[st]);
+            tma_load_4d(sb + (size_t)cc * CS * sizeof(T2), &a0.group_maps[2 * m],
+                        2 * ((ky << a0.ktl) + (k0 & ((1 << a0.ktl) - 1))), 0, k0 >> a0.ktl, cc, &bars[st]);
         if (m == 0) {
             unsigned char* gb = green0 + ((i / G) & 1) * GREEN;
             for (int gc = 0; gc < 6; ++gc)
@@ -869,9 +939,9 @@ __global__ void __launch_bounds__(3 * TX * Split<N>::TPL, sizeof(T) == 4 ? 2 : 1
         }
         gbar();
         {
-            T2* base = reinterpret_cast<T2*>(a0.group[m].spec) + comp * a0.nh + ky * a0.rs + k0 +
-                       (act ? c : 0);
-            const long long es = a0.plane;
+            T2* base = reinterpret_cast<T2*>(a0.group[m].spec) + comp * a0.nh + (k0 >> a0.ktl) * a0.kts +
+                       (ky << a0.ktl) + ((k0 + c) & ((1 << a0.ktl) - 1));
+            const int es = a0.ny << a0.ktl;
             auto st_g = [&](int pos, T2 v) { base[pos * es] = v; };
             stage_b<R2, R1, +1, TPL, false>(my, t, act, st_g);
         }
@@ -929,6 +999,34 @@ inline bool edge_supported(int n) {
     return false;
 }
 
+// the two radices of a specialised edge; false for other edges
+inline bool split_of(int n, int* r1, int* r2) {
+#define FP_CASE(N)             \
+    if (n == N) {              \
+        *r1 = Split<N>::R1;    \
+        *r2 = Split<N>::R2;    \
+        return true;           \
+    }
+    FP_FAST_EDGES(FP_CASE)
+#undef FP_CASE
+    return false;
+}
+
+// log2 of the kx tile width of the spectral layout
+inline int kt_log2(int nx) {
+#define FP_CASE(N) \
+    if (n == N) return kx_tile<N>() >= 16 ? 4 : (kx_tile<N>() >= 8 ? 3 : 2);
+    const int n = nx;
+    FP_FAST_EDGES(FP_CASE)
+#undef FP_CASE
+    return 2;
+}
+// elements of one component of the blocked spectral field
+inline long long spec_elems(int nx, int ny, int nz) {
+    const int l = kt_log2(nx);
+    return ((long long)((nx / 2 + 1 + (1 << l) - 1) >> l) << l) * ny * nz;
+}
+
 // grid rows per tile of the x passes: about 192 threads per CTA, 96 where
 // the lines are long and served by 4 threads (shared memory)
 inline int x_rows_for(int n) {
@@ -975,8 +1073,7 @@ size_t z_smem_rt(int n, int stages) {
 template <typename T, int N>
 struct Passes {
     static cudaError_t xfwd(const FastArgs& a, dim3 grid, int threads, size_t smem, cudaStream_t s);
-    static cudaError_t xinv(const FastArgs& a, int stage_bytes, dim3 grid, int threads, size_t smem,
-                            cudaStream_t s);
+    static cudaError_t xinv(const FastArgs& a, dim3 grid, int threads, size_t smem, cudaStream_t s);
     static cudaError_t y(int dir, const FastArgs& a, dim3 grid, cudaStream_t s);
     static cudaError_t z(int stages, const CUtensorMap& spec_map, const CUtensorMap& green_map,
                          const FastArgs& a, dim3 grid, size_t smem, cudaStream_t s);
@@ -990,8 +1087,7 @@ struct Passes {
 template <typename T>
 cudaError_t run_xfwd(int n, const FastArgs& a, dim3 grid, int threads, size_t smem, cudaStream_t s);
 template <typename T>
-cudaError_t run_xinv(int n, const FastArgs& a, int stage_bytes, dim3 grid, int threads, size_t smem,
-                     cudaStream_t s);
+cudaError_t run_xinv(int n, const FastArgs& a, dim3 grid, int threads, size_t smem, cudaStream_t s);
 template <typename T>
 cudaError_t run_y(int n, int dir, const FastArgs& a, dim3 grid, cudaStream_t s);
 template <typename T>

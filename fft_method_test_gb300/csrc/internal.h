@@ -22,6 +22,10 @@ struct AxisPlan {
     FftPlanDev dev{};
     double2* tw64 = nullptr;
     float2* tw32 = nullptr;
+    // stage twiddles of a specialised edge n = R1 * R2 (fft_fast.cuh), 2n
+    // entries in one allocation with tw64 / tw32; null for other edges
+    const double2* fw64 = nullptr;
+    const float2* fw32 = nullptr;
 };
 
 // Build a plan for length n (factors 2, 3, 5 only); returns false otherwise.
@@ -195,8 +199,11 @@ bool write_fvel_header(void* file, int nx, int ny, int nz, double porosity, doub
 // Computes the Green table into g64 and/or g32 (either may be null).
 cudaError_t launch_green(Problem& P, double* g64, float* g32);
 
+// elements of one component of d_spec: the [kz][ky][kx] layout of the generic
+// passes or the blocked one of the specialised passes, whichever is larger
+long long spec_capacity(const Problem& P);
 // Tensor maps of the specialised z pass (kernels_fft.cu): the spectral field
-// as [3][nz][ny][2*nxh] reals with boxes {2*tx, 1, nz, 1} and the Green table
+// blocked over kx with boxes {2*tx reals of one row, nz, 1, 1} and the Green table
 // as [6][nz][ny][nxh] with boxes {tx, 1, nz, 1}.  false when TMA is
 // unavailable or the layout does not qualify.
 bool fast_maps(Problem& P, bool dbl, int tx, const CUtensorMap** spec, const CUtensorMap** green);

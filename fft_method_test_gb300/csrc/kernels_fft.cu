@@ -87,24 +87,41 @@ bool make_axis_plan(int n, AxisPlan& p, std::string& err, cudaStream_t stream) {
     for (int i = 0; i < ns64; ++i) r64 = std::max(r64, p.dev.radix64[i]);
     p.dev.tpl32 = (n + r32 - 1) / r32;
     p.dev.tpl64 = (n + r64 - 1) / r64;
-    std::vector<double2> h64(n);
-    std::vector<float2> h32(n);
+    int r1 = 0, r2 = 0;
+    const bool special = fast::split_of(n, &r1, &r2);
+    const int entries = special ? 3 * n : n;
+    std::vector<double2> h64(entries);
+    std::vector<float2> h32(entries);
     const double two_pi = 6.283185307179586476925286766559;
     for (int j = 0; j < n; ++j) {
         const double a = two_pi * (double)j / (double)n;
         h64[j] = make_double2(std::cos(a), -std::sin(a));
         h32[j] = make_float2((float)h64[j].x, (float)h64[j].y);
     }
-    if (cudaMallocAsync(reinterpret_cast<void**>(&p.tw64), sizeof(double2) * n, stream) != cudaSuccess ||
-        cudaMallocAsync(reinterpret_cast<void**>(&p.tw32), sizeof(float2) * n, stream) != cudaSuccess) {
+    if (special) {  // [k < R1][a < R2] forward, [k < R2][a < R1] inverse: roots a * k < n
+        for (int k = 0; k < r1; ++k)
+            for (int a = 0; a < r2; ++a) {
+                const int f = n + k * r2 + a, i = 2 * n + a * r1 + k;
+                h64[f] = h64[a * k];
+                h32[f] = h32[a * k];
+                h64[i] = make_double2(h64[a * k].x, -h64[a * k].y);
+                h32[i] = make_float2(h32[a * k].x, -h32[a * k].y);
+            }
+    }
+    if (cudaMallocAsync(reinterpret_cast<void**>(&p.tw64), sizeof(double2) * entries, stream) != cudaSuccess ||
+        cudaMallocAsync(reinterpret_cast<void**>(&p.tw32), sizeof(float2) * entries, stream) != cudaSuccess) {
         err = "device allocation failed for FFT twiddles";
         return false;
     }
-    cudaMemcpyAsync(p.tw64, h64.data(), sizeof(double2) * n, cudaMemcpyHostToDevice, stream);
-    cudaMemcpyAsync(p.tw32, h32.data(), sizeof(float2) * n, cudaMemcpyHostToDevice, stream);
+    cudaMemcpyAsync(p.tw64, h64.data(), sizeof(double2) * entries, cudaMemcpyHostToDevice, stream);
+    cudaMemcpyAsync(p.tw32, h32.data(), sizeof(float2) * entries, cudaMemcpyHostToDevice, stream);
     cudaStreamSynchronize(stream);  // the host tables must outlive their copies
     p.dev.tw64 = p.tw64;
     p.dev.tw32 = p.tw32;
+    if (special) {
+        p.fw64 = p.tw64 + n;
+        p.fw32 = p.tw32 + n;
+    }
     return true;
 }
 
@@ -113,6 +130,8 @@ void free_axis_plan(AxisPlan& p, cudaStream_t stream) {
     if (p.tw32) cudaFreeAsync(p.tw32, stream);
     p.tw64 = nullptr;
     p.tw32 = nullptr;
+    p.fw64 = nullptr;
+    p.fw32 = nullptr;
 }
 
 // ---------------------------------------------------------------------------
@@ -203,6 +222,10 @@ static bool tma_setup(Problem& P, bool dbl, int axis, int tpl, int padsh, TmaTil
     return true;
 }
 
+long long spec_capacity(const Problem& P) {
+    return std::max(P.nh, fast::spec_elems(P.nx, P.ny, P.nz));
+}
+
 bool fast_maps(Problem& P, bool dbl, int tx, const CUtensorMap** spec, const CUtensorMap** green) {
     if (!tma_encoder()) return false;
     const int k = dbl ? 0 : 1;
@@ -212,11 +235,14 @@ bool fast_maps(Problem& P, bool dbl, int tx, const CUtensorMap** spec, const CUt
         const size_t e = dbl ? sizeof(double) : sizeof(float);
         const CUtensorMapDataType dt = dbl ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
         const cuuint32_t estr[4] = {1, 1, 1, 1};
-        // the spectral field: interleaved (re, im) reals
-        const cuuint64_t sd[4] = {(cuuint64_t)(2 * P.nxh), (cuuint64_t)P.ny, (cuuint64_t)P.nz, 3};
-        const cuuint64_t ss[3] = {(cuuint64_t)(2 * P.rs * e), (cuuint64_t)(2 * P.rs * P.ny * e),
-                                  (cuuint64_t)(2 * P.nh * e)};
-        const cuuint32_t sb[4] = {(cuuint32_t)(2 * tx), 1u, (cuuint32_t)P.nz, 1u};
+        // the spectral field, interleaved (re, im) reals, blocked over kx
+        // tiles (fft_fast.cuh): one row of ny * kt elements per (kx tile, kz)
+        const int ktl = fast::kt_log2(P.nx);
+        const long long nhs = fast::spec_elems(P.nx, P.ny, P.nz);
+        const cuuint64_t row = (cuuint64_t)(2 * P.ny) << ktl;
+        const cuuint64_t sd[4] = {row, (cuuint64_t)P.nz, (cuuint64_t)((P.nxh + (1 << ktl) - 1) >> ktl), 3};
+        const cuuint64_t ss[3] = {row * e, row * P.nz * e, (cuuint64_t)(2 * nhs * e)};
+        const cuuint32_t sb[4] = {(cuuint32_t)(2 * tx), (cuuint32_t)P.nz, 1u, 1u};
         CUresult r = tma_encoder()(&P.fz_spec_map[k], dt, 4, P.d_spec, sd, ss, sb, estr,
                                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                                    CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
