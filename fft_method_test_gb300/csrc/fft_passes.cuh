@@ -90,6 +90,7 @@ struct TmaTile {
 
 template <typename T, int SRC>
 __global__ void __launch_bounds__(256, 3) k_xfwd(XArgs a) {
+    pdl_wait();
     if (a.skip && *a.skip) return;
     using T2 = c_t<T>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -191,6 +192,7 @@ __global__ void __launch_bounds__(256, 3) k_xfwd(XArgs a) {
                                             NoDst<T2>{});
     }
 
+    if (sizeof(T) == 4) pdl_trigger();
     // 4) separate the two real spectra and store the half spectrum
     const int nxh = a.nxh;
     const int tot2 = nq * nxh;
@@ -237,6 +239,7 @@ struct ColIo {
 
 template <typename T, int S>
 __device__ __forceinline__ void ypass_body(const YArgs& a) {
+    pdl_wait();
     if (a.skip && *a.skip) return;
     using T2 = c_t<T>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -379,6 +382,7 @@ __device__ __forceinline__ void z_fused_rt(const ZArgs& a, c_t<T>* const* sl, Sr
 // 2 = inverse z only
 template <typename T, int ZMODE>
 __device__ __forceinline__ void zgreen_body(const ZArgs& a) {
+    pdl_wait();
     if (a.skip && *a.skip) return;
     using T2 = c_t<T>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -453,6 +457,7 @@ struct RawIo {
 template <typename T, int S>
 __global__ void __launch_bounds__(256) k_ypass_tma(const __grid_constant__ CUtensorMap map, YArgs a,
                                                    TmaTile tt) {
+    pdl_wait();
     if (a.skip && *a.skip) return;
     using T2 = c_t<T>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -508,6 +513,7 @@ __global__ void __launch_bounds__(256) k_ypass_tma(const __grid_constant__ CUten
 template <typename T>
 __global__ void __launch_bounds__(256) k_zgreen_tma(const __grid_constant__ CUtensorMap map, ZArgs a,
                                                     TmaTile tt) {
+    pdl_wait();
     if (a.skip && *a.skip) return;
     using T2 = c_t<T>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -681,6 +687,7 @@ struct SmemRows {
 
 template <typename T, int DST>
 __global__ void __launch_bounds__(256, 3) k_xinv(XArgs a) {
+    pdl_wait();
     if (a.skip && *a.skip) return;
     using T2 = c_t<T>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -706,6 +713,7 @@ __global__ void __launch_bounds__(256, 3) k_xinv(XArgs a) {
 // deterministic).  smem: 128 B barriers | raw[2] | lines.
 template <typename T, int DST>
 __global__ void __launch_bounds__(256, 2) k_xinv_bulk(XArgs a, int raw_bytes) {
+    pdl_wait();
     if (a.skip && *a.skip) return;
     using T2 = c_t<T>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -806,8 +814,7 @@ inline void ensure_max_smem(K kern, std::atomic<unsigned long long>& done) {
     do {                                                          \
         static std::atomic<unsigned long long> smem_set_{0};      \
         ensure_max_smem(kern, smem_set_);                         \
-        FP_LAUNCHED();                                            \
-        kern<<<grid, threads, smem, s>>>(__VA_ARGS__);            \
+        launch_pdl(kern, grid, threads, smem, s, __VA_ARGS__);    \
     } while (0)
 
 #ifdef FP_DEFINE_X_RUNNERS

@@ -113,7 +113,7 @@ cudaError_t group_iterations(Problem* const* m, int members, int count, GroupTab
         }
     }
     const int nparts = (int)geom0[7];  // partial rows of the inverse x pass
-    int max_blocks = 1;
+    int max_blocks = 1, threads = 0;
     for (int i = 0; i < count; ++i) {
         for (int p = 0; p < members; ++p) {
             IterArgs ia;
@@ -126,9 +126,12 @@ cudaError_t group_iterations(Problem* const* m, int members, int count, GroupTab
             fa.dst = aa.dst;
             fa.dot_with = aa.dot_with;
             fa.skip = aa.skip;
+            fa.alpha_sc = aa.alpha_sc;
+            fa.alpha_ticket = aa.alpha_ticket;
             t->h_fast[(size_t)i * members + p] = fa;
             t->h_iter[(size_t)i * members + p] = ia;
             max_blocks = std::max(max_blocks, ia.nblk);
+            threads = ia.threads;
         }
     }
     const size_t nf = (size_t)count * members;
@@ -146,7 +149,7 @@ cudaError_t group_iterations(Problem* const* m, int members, int count, GroupTab
         e = fast_apply_group(P0, prec, members, t->d_fast + (size_t)i * members, t->d_maps, shared_green,
                              &np);
         if (e != cudaSuccess) return e;
-        e = group_iteration_tail(s, t->d_iter + (size_t)i * members, members, max_blocks);
+        e = group_iteration_tail(s, t->d_iter + (size_t)i * members, members, max_blocks, threads);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;

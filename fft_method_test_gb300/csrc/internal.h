@@ -44,7 +44,7 @@ struct MinresScalars {
     double phi_bar;
     double rel_res;
     // coefficients of the current iteration's vector update
-    double eps, delta, rho, step, inv_beta_new;
+    double eps, delta, inv_rho, step, inv_beta_new;
     double vsum[3];  // component sums of the current Lanczos vector v
     double zmean[3];
     long long it;     // completed iterations
@@ -164,7 +164,7 @@ struct Problem {
 
 constexpr int kMaxPartials = 8192;
 // d_red slot (in doubles) holding the block-count tickets of the fused MINRES
-// vector kernels (two unsigned ints, zero between launches)
+// kernels (z update, v/w update, alpha: three unsigned ints, zero between launches)
 constexpr int kTicketSlot = 56;
 
 // ---- setup kernels (kernels_setup.cu) ----
@@ -241,6 +241,10 @@ struct ApplyArgs {
     const int* skip = nullptr;       // device flag: when nonzero every pass returns at once
     int precision = -1;              // kFP64 / kMixed; -1 = the problem's default
     int stage = kStageFull;
+    // specialised passes: the last block of the inverse x pass computes the z
+    // mean and alpha from the partial rows (both set, or both null)
+    MinresScalars* alpha_sc = nullptr;
+    unsigned int* alpha_ticket = nullptr;
 };
 
 // Runs the five passes (forward x, y, z + Green + inverse z, inverse y,
@@ -248,6 +252,8 @@ struct ApplyArgs {
 // P.d_partials as [blocks][4] = {sum_x, sum_y, sum_z, dot}; returns the number
 // of partial rows in *nparts.
 cudaError_t launch_apply(Problem& P, const ApplyArgs& a, int* nparts);
+// true when launch_apply runs the specialised passes (fast_dispatch.cu)
+bool fast_apply_supported(const Problem& P, int precision, int src_kind, int dst_kind, int stage);
 
 // ---- groups of problems of one grid (kernels_minres.cu, group.cu) ----
 // One member's pointers for one MINRES iteration of a group: the group
@@ -257,6 +263,7 @@ struct IterArgs {
     double* partials;  // the apply's partial rows in, the vector kernels' out
     int nparts;        // partial rows the apply wrote
     int nblk;          // vector-kernel blocks of this member
+    int threads;       // and threads per block (one value for a grid)
     double inv_nb;
     long long nb;
     double* z;
@@ -266,15 +273,15 @@ struct IterArgs {
     double* w_prev;
     const double* w;
     double* x;
-    unsigned int* tickets;  // [0] z update, [1] v/w update
+    unsigned int* tickets;  // [0] z update, [1] v/w update, [2] alpha
     double* hist;
 };
 // Arguments of the next iteration of P (the buffer rotation at P.queued, which
 // it advances) and the apply it starts with.
 cudaError_t iteration_args(Problem& P, IterArgs* t, ApplyArgs* aa);
-// alpha, z update (+ Givens step), v/w/x update (+ iteration end) of
-// `members` problems, one launch each; max_blocks = the largest nblk.
-cudaError_t group_iteration_tail(cudaStream_t s, const IterArgs* d_tab, int members, int max_blocks);
+// z update (+ Givens step), v/w/x update (+ iteration end) of `members`
+// problems, one launch each; max_blocks = the largest nblk.
+cudaError_t group_iteration_tail(cudaStream_t s, const IterArgs* d_tab, int members, int max_blocks, int threads);
 
 // Device tables of a group's lockstep iterations (group.cu).
 struct GroupTables;
@@ -291,9 +298,10 @@ cudaError_t group_iterations(Problem* const* m, int members, int count, GroupTab
 cudaError_t launch_sum3(Problem& P, const double* v, long long nb, double* out3);
 // Reduce [nparts][4] partials into out4 (deterministic, one block).
 cudaError_t launch_reduce4(Problem& P, int nparts, double* out4);
-// r0_precision: operator precision of r0 = b - A x0 (-1: the problem's own)
+// r0_precision: operator precision of r0 = b - A x0 (-1: the problem's own);
+// ax0: A x0 with its mean removed where the caller has it, or null
 cudaError_t minres_start(Problem& P, const double* b, const double* x0, double tol,
-                         long long maxit, int r0_precision = -1);
+                         long long maxit, int r0_precision = -1, const double* ax0 = nullptr);
 cudaError_t minres_iteration(Problem& P);
 cudaError_t minres_iterations(Problem& P, int count);
 void release_graphs(Problem& P);

@@ -2,15 +2,16 @@
 //
 // All Lanczos vectors, inner products and the Givens recurrence stay in FP64
 // on the GPU.  One iteration is
-//   apply   z_raw = A_raw v, fused partial sums of z_raw and of v . z_raw
-//   alpha   one CTA: z mean, alpha = v . (z_raw - mean)
+//   apply   z_raw = A_raw v, fused partial sums of z_raw and of v . z_raw;
+//   alpha   z mean, alpha = v . (z_raw - mean): the last block of the
+//           specialised inverse x pass, or one CTA after the generic passes
 //   zupd    z = (z_raw - mean) - (alpha v + beta v_old), partial |z|^2
-//   scalar  one CTA: beta_new, Givens rotation, phi_bar, residual history,
-//           stop test (the reference's order of operations)
+//   scalar  its last block: beta_new, Givens rotation, phi_bar, residual
+//           history, stop test (the reference's order of operations)
 //   vwupd   v_new = z / beta_new, w_next = (v - eps w_prev - delta w) / rho,
 //           x += (cs_new phi_bar) w_next, partial component sums of v_new
-//   finish  one CTA: component sums of v_new (the next apply's input mean),
-//           iteration counter, stop -> done
+//   finish  its last block: component sums of v_new (the next apply's input
+//           mean), iteration counter, stop -> done
 // Kernels return at once when the solve is done, so the host can queue
 // iterations ahead and read the scalar block only every few iterations.
 #include <cuda_runtime.h>
@@ -20,6 +21,7 @@
 
 #include "common.cuh"
 #include "internal.h"
+#include "minres_device.cuh"
 
 namespace fp {
 
@@ -28,12 +30,20 @@ namespace {
 constexpr int kVecThreads = 256;
 constexpr double kBreakdownEps = 1e-14;
 
-int vec_blocks(const Problem& P, long long m) {
-    long long b = (m + kVecThreads - 1) / kVecThreads;
+int vec_blocks(const Problem& P, long long m, int threads = kVecThreads) {
+    long long b = (m + threads - 1) / threads;
     const long long cap = 8LL * (P.sm_count > 0 ? P.sm_count : 152);
     if (b > cap) b = cap;
     if (b < 1) b = 1;
     return (int)b;
+}
+
+// Threads per block of the z and v/w updates: FP64 bounds them, so the small
+// grids' few thousand voxel pairs go to all SMs in small blocks (64^3: 29 k
+// support voxels are 57 blocks of 256 threads or 228 of 64).  By the grid, not
+// the support, so that the members of a group share it.
+int iter_threads(const Problem& P) {
+    return P.n <= 80LL * 80 * 80 ? 64 : (P.n <= 128LL * 128 * 128 ? 128 : kVecThreads);
 }
 
 // partial component sums (and with SQUARES the sum of squares; GB300's FP64
@@ -42,7 +52,8 @@ int vec_blocks(const Problem& P, long long m) {
 // the component of every load static; the odd tail voxel goes to the first
 // thread of block 0.
 template <bool SQUARES>
-__global__ void k_sum3(const double* __restrict__ v, long long nb, double* partials) {
+__global__ void k_sum3(const double* v, long long nb, double* partials) {
+    pdl_wait();
     __shared__ double red[4 * 32];
     double acc[4] = {0, 0, 0, 0};
     const long long npair = nb >> 1;
@@ -70,48 +81,28 @@ __global__ void k_sum3(const double* __restrict__ v, long long nb, double* parti
         for (int i = 0; i < 4; ++i) partials[4LL * blockIdx.x + i] = out[i];
 }
 
-__global__ void k_reduce4(const double* __restrict__ partials, int nparts, double* out) {
+__global__ void k_reduce4(const double* partials, int nparts, double* out) {
+    pdl_wait();
     __shared__ double red[4 * 32];
-    double acc[4] = {0, 0, 0, 0};
-    for (int i = threadIdx.x; i < nparts; i += blockDim.x)
-        for (int j = 0; j < 4; ++j) acc[j] += partials[4LL * i + j];
     double o[4];
-    block_sum<4>(acc, red, o);
+    sum_rows<4, 4>(partials, nparts, red, o);
     if (threadIdx.x == 0)
         for (int j = 0; j < 4; ++j) out[j] = o[j];
 }
 
 // ---- iteration kernels ------------------------------------------------------
 
-__device__ __forceinline__ void alpha_body(MinresScalars* sc, const double* __restrict__ partials,
-                                           int nparts, double inv_nb) {
-    if (sc->done) return;
-    __shared__ double red[4 * 32];
-    double acc[4] = {0, 0, 0, 0};
-    for (int i = threadIdx.x; i < nparts; i += blockDim.x)
-        for (int j = 0; j < 4; ++j) acc[j] += partials[4LL * i + j];
-    double o[4];
-    block_sum<4>(acc, red, o);
-    if (threadIdx.x == 0) {
-        double corr = 0.0;
-        for (int c = 0; c < 3; ++c) {
-            sc->zmean[c] = o[c] * inv_nb;
-            corr += sc->zmean[c] * sc->vsum[c];
-        }
-        sc->alpha = o[3] - corr;
-    }
-}
-
-__global__ void k_alpha(MinresScalars* sc, const double* __restrict__ partials, int nparts,
+__global__ void k_alpha(MinresScalars* sc, const double* partials, int nparts,
                         double inv_nb) {
-    alpha_body(sc, partials, nparts, inv_nb);
+    pdl_wait();
+    __shared__ double red[4 * 32];
+    alpha_body(sc, partials, nparts, inv_nb, red);
 }
 
 __device__ void scalar_step(MinresScalars* sc, const double* __restrict__ partials, int nparts,
                             double* hist, double* red);
 __device__ void finish_step(MinresScalars* sc, const double* __restrict__ partials, int nparts,
                             double* red);
-__device__ __forceinline__ bool last_block(unsigned int* counter, unsigned int nblk);
 
 // Two voxels (six doubles, three aligned double2) per thread: components are
 // static, loads are 16-byte vectors.  The odd tail voxel is handled by the
@@ -158,48 +149,57 @@ __device__ __forceinline__ void zupd_body(MinresScalars* sc, double* __restrict_
     if (last_block(counter, nblk)) scalar_step(sc, partials, (int)nblk, hist, red);
 }
 
-__global__ void k_zupd(MinresScalars* sc, double* __restrict__ z, const double* __restrict__ v,
-                       const double* __restrict__ v_old, long long nb, double* partials,
+__global__ void k_zupd(MinresScalars* sc, double* z, const double* v,
+                       const double* v_old, long long nb, double* partials,
                        unsigned int* counter, double* hist) {
+    pdl_wait();
     zupd_body(sc, z, v, v_old, nb, partials, counter, hist, blockIdx.x, gridDim.x);
 }
 
 // The Givens step of one iteration from the |z|^2 partials, run by one whole
 // block (the last block of k_zupd): beta_new, the rotation, phi_bar, the
 // residual history and the stop test (MinresSolver.cpp:148-186).
+// The FP64 pipe issues a warp instruction every 16 clocks per SM, so the step's
+// length is its number of FP64 instructions: the four quotients are one
+// division of four lanes, and rho is a square root (hypot where the squares
+// could leave the range).
 __device__ void scalar_step(MinresScalars* sc, const double* __restrict__ partials, int nparts,
                             double* hist, double* red) {
-    double acc[1] = {0.0};
-    for (int i = threadIdx.x; i < nparts; i += blockDim.x) acc[0] += __ldcg(partials + i);
     double o[1];
-    block_sum<1>(acc, red, o);
-    if (threadIdx.x != 0) return;
+    sum_rows<1, 1>(partials, nparts, red, o);
+    if (threadIdx.x >= 32) return;
+    const int lane = threadIdx.x;
     const double beta_new = sqrt(o[0] > 0.0 ? o[0] : 0.0);
     const double alpha = sc->alpha;
     const double beta = sc->beta;
+    const double phi_bar = sc->phi_bar, cs_old = sc->cs_old, sn_old = sc->sn_old, cs = sc->cs, sn = sc->sn;
     // MinresSolver.cpp:148-186
-    const double eps = sc->sn_old * beta;
-    const double delta_raw = -sc->cs_old * beta;
-    const double delta = sc->cs * delta_raw + sc->sn * alpha;
-    const double phi = sc->sn * delta_raw - sc->cs * alpha;
-    const double rho = hypot(phi, beta_new);
-    double cs_new = 1.0, sn_new = 0.0;
-    if (rho > kBreakdownEps) {
-        cs_new = phi / rho;
-        sn_new = beta_new / rho;
-    }
+    const double delta_raw = -cs_old * beta;
+    const double phi = sn * delta_raw - cs * alpha;
+    const double r2 = phi * phi + beta_new * beta_new;
+    const double rho = r2 > 1e-280 && r2 < 1e280 ? sqrt(r2) : hypot(phi, beta_new);
+    // cs = phi / rho, sn = beta_new / rho, 1 / rho, 1 / beta_new
+    const double quot = (lane == 0 ? phi : (lane == 1 ? beta_new : 1.0)) / (lane < 3 ? rho : beta_new);
+    const bool rb = rho > kBreakdownEps;
+    const double cs_new = rb ? __shfl_sync(0xffffffffu, quot, 0) : 1.0;
+    const double sn_new = rb ? __shfl_sync(0xffffffffu, quot, 1) : 0.0;
+    const double inv_rho = rb ? __shfl_sync(0xffffffffu, quot, 2) : 0.0;
+    const double inv_beta = beta_new > kBreakdownEps ? __shfl_sync(0xffffffffu, quot, 3) : 0.0;
+    if (lane != 0) return;
+    const double phi_bar_new = phi_bar * sn_new;
     sc->beta_new = beta_new;
-    sc->eps = eps;
-    sc->delta = delta;
-    sc->rho = rho;
-    sc->step = cs_new * sc->phi_bar;
-    sc->phi_bar *= sn_new;
-    sc->cs_old = sc->cs;
-    sc->sn_old = sc->sn;
+    sc->eps = sn_old * beta;
+    sc->delta = cs * delta_raw + sn * alpha;
+    sc->inv_rho = inv_rho;
+    sc->inv_beta_new = inv_beta;
+    sc->step = cs_new * phi_bar;
+    sc->phi_bar = phi_bar_new;
+    sc->cs_old = cs;
+    sc->sn_old = sn;
     sc->cs = cs_new;
     sc->sn = sn_new;
     sc->beta = beta_new;
-    const double rel = fabs(sc->phi_bar) / sc->rhs_norm;
+    const double rel = fabs(phi_bar_new) / sc->rhs_norm;
     sc->rel_res = rel;
     const long long k = sc->it + 1;
     if (hist) hist[k] = rel;
@@ -222,15 +222,11 @@ __device__ __forceinline__ void vwupd_body(MinresScalars* sc, const double* __re
                                            unsigned int blk, unsigned int nblk) {
     if (sc->done) return;
     __shared__ double red[4 * 32];
-    const double beta_new = sc->beta_new, eps = sc->eps, delta = sc->delta, rho = sc->rho;
-    const double step = sc->step;
-    const bool vb = beta_new > kBreakdownEps;
-    const bool rb = rho > kBreakdownEps;
-    // one division per CTA: GB300's FP64 pipe is narrow, and per-element
-    // divisions made this kernel FP64-bound (x / d becomes x * (1 / d), a
-    // difference of at most one rounding)
-    const double inv_beta = vb ? 1.0 / beta_new : 0.0;
-    const double inv_rho = rb ? 1.0 / rho : 0.0;
+    const double eps = sc->eps, delta = sc->delta, step = sc->step;
+    // reciprocals formed once per iteration by the scalar step: GB300's FP64
+    // pipe bounds this kernel, and a division in every thread of every block
+    // cost as much as the update of three elements
+    const double inv_beta = sc->inv_beta_new, inv_rho = sc->inv_rho;
     double acc[4] = {0, 0, 0, 0};
     const long long npair = nb >> 1;
     const double2* z2 = reinterpret_cast<const double2*>(z);
@@ -275,27 +271,25 @@ __device__ __forceinline__ void vwupd_body(MinresScalars* sc, const double* __re
     if (last_block(counter, nblk)) finish_step(sc, partials, (int)nblk, red);
 }
 
-__global__ void k_vwupd(MinresScalars* sc, const double* __restrict__ z, const double* __restrict__ v,
-                        double* __restrict__ v_new, double* __restrict__ w_prev_to_next,
-                        const double* __restrict__ w, double* __restrict__ x, long long nb,
+__global__ void k_vwupd(MinresScalars* sc, const double* z, const double* v,
+                        double* v_new, double* w_prev_to_next,
+                        const double* w, double* x, long long nb,
                         double* partials, unsigned int* counter) {
+    pdl_wait();
     vwupd_body(sc, z, v, v_new, w_prev_to_next, w, x, nb, partials, counter, blockIdx.x, gridDim.x);
 }
 
 // ---- group kernels: one launch for several problems (tab[member]) ------------
 
-__global__ void k_alpha_g(const IterArgs* __restrict__ tab) {
-    const IterArgs& t = tab[blockIdx.x];
-    alpha_body(t.sc, t.partials, t.nparts, t.inv_nb);
-}
-
-__global__ void k_zupd_g(const IterArgs* __restrict__ tab) {
+__global__ void k_zupd_g(const IterArgs* tab) {
+    pdl_wait();
     const IterArgs& t = tab[blockIdx.y];
     if (blockIdx.x >= (unsigned)t.nblk) return;
     zupd_body(t.sc, t.z, t.v, t.v_old, t.nb, t.partials, t.tickets, t.hist, blockIdx.x, t.nblk);
 }
 
-__global__ void k_vwupd_g(const IterArgs* __restrict__ tab) {
+__global__ void k_vwupd_g(const IterArgs* tab) {
+    pdl_wait();
     const IterArgs& t = tab[blockIdx.y];
     if (blockIdx.x >= (unsigned)t.nblk) return;
     vwupd_body(t.sc, t.z, t.v, t.v_new, t.w_prev, t.w, t.x, t.nb, t.partials, t.tickets + 1, blockIdx.x,
@@ -307,11 +301,8 @@ __global__ void k_vwupd_g(const IterArgs* __restrict__ tab) {
 // iteration counter, stop -> done.
 __device__ void finish_step(MinresScalars* sc, const double* __restrict__ partials, int nparts,
                             double* red) {
-    double acc[4] = {0, 0, 0, 0};
-    for (int i = threadIdx.x; i < nparts; i += blockDim.x)
-        for (int j = 0; j < 4; ++j) acc[j] += __ldcg(partials + 4LL * i + j);
     double o[4];
-    block_sum<4>(acc, red, o);
+    sum_rows<4, 4>(partials, nparts, red, o);
     if (threadIdx.x == 0) {
         for (int c = 0; c < 3; ++c) sc->vsum[c] = o[c];
         sc->it += 1;
@@ -319,31 +310,14 @@ __device__ void finish_step(MinresScalars* sc, const double* __restrict__ partia
     }
 }
 
-// true in every thread of the block that finishes last among the nblk blocks
-// of one problem (its partial sums are then all in memory); the counter is reset
-__device__ __forceinline__ bool last_block(unsigned int* counter, unsigned int nblk) {
-    __shared__ bool last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const unsigned int t = atomicAdd(counter, 1u);
-        last = t == nblk - 1;
-        if (last) *counter = 0u;
-    }
-    __syncthreads();
-    return last;
-}
-
 // ---- start-up kernels -------------------------------------------------------
 
-__global__ void k_start_norms(MinresScalars* sc, const double* __restrict__ partials, int nparts,
+__global__ void k_start_norms(MinresScalars* sc, const double* partials, int nparts,
                               int which) {
+    pdl_wait();
     __shared__ double red[4 * 32];
-    double acc[4] = {0, 0, 0, 0};
-    for (int i = threadIdx.x; i < nparts; i += blockDim.x)
-        for (int j = 0; j < 4; ++j) acc[j] += partials[4LL * i + j];
     double o[4];
-    block_sum<4>(acc, red, o);
+    sum_rows<4, 4>(partials, nparts, red, o);
     if (threadIdx.x == 0) {
         const double nrm = sqrt(o[3] > 0.0 ? o[3] : 0.0);
         if (which == 0) {
@@ -355,9 +329,10 @@ __global__ void k_start_norms(MinresScalars* sc, const double* __restrict__ part
 }
 
 // r0 = b - (A x0 - mean) when have_x0, else b.
-__global__ void k_residual0(const MinresScalars* sc, const double* __restrict__ b,
-                            double* __restrict__ z, const double* __restrict__ zmean3,
+__global__ void k_residual0(const MinresScalars* sc, const double* b,
+                            double* z, const double* zmean3,
                             long long m, int have_x0) {
+    pdl_wait();
     const double m0 = have_x0 ? zmean3[0] : 0.0, m1 = have_x0 ? zmean3[1] : 0.0,
                  m2 = have_x0 ? zmean3[2] : 0.0;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < m;
@@ -372,43 +347,50 @@ __global__ void k_residual0(const MinresScalars* sc, const double* __restrict__ 
     }
 }
 
-__global__ void k_scale_div(const double* __restrict__ z, double* __restrict__ v,
+__global__ void k_scale_div(const double* z, double* v,
                             const MinresScalars* sc, long long m) {
+    pdl_wait();
     const double beta = sc->beta;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < m;
          i += (long long)gridDim.x * blockDim.x)
         v[i] = z[i] / beta;
 }
 
-__global__ void k_zmean_from_partials(const double* __restrict__ partials, int nparts,
+__global__ void k_zmean_from_partials(const double* partials, int nparts,
                                       double inv_nb, double* out3) {
+    pdl_wait();
     __shared__ double red[4 * 32];
-    double acc[4] = {0, 0, 0, 0};
-    for (int i = threadIdx.x; i < nparts; i += blockDim.x)
-        for (int j = 0; j < 4; ++j) acc[j] += partials[4LL * i + j];
     double o[4];
-    block_sum<4>(acc, red, o);
+    sum_rows<4, 4>(partials, nparts, red, o);
     if (threadIdx.x == 0)
         for (int c = 0; c < 3; ++c) out3[c] = o[c] * inv_nb;
+}
+
+__global__ void k_axpby(double* out, double a, const double* x, double b,
+                        const double* y, long long m) {
+    pdl_wait();
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < m;
+         i += (long long)gridDim.x * blockDim.x)
+        out[i] = a * x[i] + b * y[i];
 }
 
 }  // namespace
 
 cudaError_t launch_sum3(Problem& P, const double* v, long long nb, double* out4) {
     const int blocks = vec_blocks(P, (nb + 1) / 2);
-    FP_LAUNCHED(); k_sum3<false><<<blocks, kVecThreads, 0, P.stream>>>(v, nb, P.d_partials);
-    FP_LAUNCHED(); k_reduce4<<<1, 256, 0, P.stream>>>(P.d_partials, blocks, out4);
+    launch_pdl(k_sum3<false>, blocks, kVecThreads, 0, P.stream, v, nb, P.d_partials);
+    launch_pdl(k_reduce4, 1, 256, 0, P.stream, P.d_partials, blocks, out4);
     return cudaGetLastError();
 }
 
 cudaError_t launch_reduce4(Problem& P, int nparts, double* out4) {
-    FP_LAUNCHED(); k_reduce4<<<1, 512, 0, P.stream>>>(P.d_partials, nparts, out4);
+    launch_pdl(k_reduce4, 1, 512, 0, P.stream, P.d_partials, nparts, out4);
     return cudaGetLastError();
 }
 
 
 cudaError_t minres_start(Problem& P, const double* b, const double* x0, double tol,
-                         long long maxit, int r0_precision) {
+                         long long maxit, int r0_precision, const double* ax0) {
     const long long m = 3 * P.nb;
     MinresScalars init{};
     init.tol = tol;
@@ -422,11 +404,15 @@ cudaError_t minres_start(Problem& P, const double* b, const double* x0, double t
     if (e != cudaSuccess) return e;
     const int blocks = vec_blocks(P, m);
     // |b|
-    FP_LAUNCHED(); k_sum3<true><<<blocks, kVecThreads, 0, P.stream>>>(b, P.nb, P.d_partials);
-    FP_LAUNCHED(); k_start_norms<<<1, 256, 0, P.stream>>>(P.d_sc, P.d_partials, blocks, 0);
+    launch_pdl(k_sum3<true>, blocks, kVecThreads, 0, P.stream, b, P.nb, P.d_partials);
+    launch_pdl(k_start_norms, 1, 256, 0, P.stream, P.d_sc, P.d_partials, blocks, 0);
     // x = x0 or 0
     if (x0) {
         cudaMemcpyAsync(P.d_x, x0, sizeof(double) * m, cudaMemcpyDeviceToDevice, P.stream);
+    }
+    if (x0 && ax0) {
+        launch_pdl(k_axpby, blocks, kVecThreads, 0, P.stream, P.d_z, 1.0, b, -1.0, ax0, m);
+    } else if (x0) {
         // z_raw = A_raw x0 with input mean removal
         launch_sum3(P, P.d_x, P.nb, P.d_red);
         ApplyArgs a;
@@ -439,16 +425,16 @@ cudaError_t minres_start(Problem& P, const double* b, const double* x0, double t
         int nparts = 0;
         e = launch_apply(P, a, &nparts);
         if (e != cudaSuccess) return e;
-        FP_LAUNCHED(); k_zmean_from_partials<<<1, 512, 0, P.stream>>>(P.d_partials, nparts, 1.0 / (double)P.nb,
+        launch_pdl(k_zmean_from_partials, 1, 512, 0, P.stream, P.d_partials, nparts, 1.0 / (double)P.nb,
                                                        P.d_red + 4);
-        FP_LAUNCHED(); k_residual0<<<blocks, kVecThreads, 0, P.stream>>>(P.d_sc, b, P.d_z, P.d_red + 4, m, 1);
+        launch_pdl(k_residual0, blocks, kVecThreads, 0, P.stream, P.d_sc, b, P.d_z, P.d_red + 4, m, 1);
     } else {
         cudaMemsetAsync(P.d_x, 0, sizeof(double) * m, P.stream);
-        FP_LAUNCHED(); k_residual0<<<blocks, kVecThreads, 0, P.stream>>>(P.d_sc, b, P.d_z, nullptr, m, 0);
+        launch_pdl(k_residual0, blocks, kVecThreads, 0, P.stream, P.d_sc, b, P.d_z, nullptr, m, 0);
     }
     // beta1 = |r0|
-    FP_LAUNCHED(); k_sum3<true><<<blocks, kVecThreads, 0, P.stream>>>(P.d_z, P.nb, P.d_partials);
-    FP_LAUNCHED(); k_start_norms<<<1, 256, 0, P.stream>>>(P.d_sc, P.d_partials, blocks, 1);
+    launch_pdl(k_sum3<true>, blocks, kVecThreads, 0, P.stream, P.d_z, P.nb, P.d_partials);
+    launch_pdl(k_start_norms, 1, 256, 0, P.stream, P.d_sc, P.d_partials, blocks, 1);
     e = cudaMemcpyAsync(P.h_sc, P.d_sc, sizeof(MinresScalars), cudaMemcpyDeviceToHost, P.stream);
     if (e != cudaSuccess) return e;
     e = cudaStreamSynchronize(P.stream);
@@ -485,13 +471,13 @@ cudaError_t minres_start(Problem& P, const double* b, const double* x0, double t
     *P.h_sc = s;
     cudaMemcpyAsync(P.d_sc, P.h_sc, sizeof(MinresScalars), cudaMemcpyHostToDevice, P.stream);
     // v = r0 / beta1 into V[0]; v_old = V[2] = 0; w = 0
-    FP_LAUNCHED(); k_scale_div<<<blocks, kVecThreads, 0, P.stream>>>(P.d_z, P.d_v[0], P.d_sc, m);
+    launch_pdl(k_scale_div, blocks, kVecThreads, 0, P.stream, P.d_z, P.d_v[0], P.d_sc, m);
     cudaMemsetAsync(P.d_v[2], 0, sizeof(double) * m, P.stream);
     cudaMemsetAsync(P.d_w[0], 0, sizeof(double) * m, P.stream);
     cudaMemsetAsync(P.d_w[1], 0, sizeof(double) * m, P.stream);
     // component sums of v (input mean of the first apply)
-    FP_LAUNCHED(); k_sum3<false><<<blocks, kVecThreads, 0, P.stream>>>(P.d_v[0], P.nb, P.d_partials);
-    FP_LAUNCHED(); k_reduce4<<<1, 256, 0, P.stream>>>(P.d_partials, blocks, P.d_red + 8);
+    launch_pdl(k_sum3<false>, blocks, kVecThreads, 0, P.stream, P.d_v[0], P.nb, P.d_partials);
+    launch_pdl(k_reduce4, 1, 256, 0, P.stream, P.d_partials, blocks, P.d_red + 8);
     // copy the three sums into sc->vsum
     cudaMemcpyAsync(&P.d_sc->vsum[0], P.d_red + 8, sizeof(double) * 3, cudaMemcpyDeviceToDevice,
                     P.stream);
@@ -579,7 +565,8 @@ cudaError_t iteration_args(Problem& P, IterArgs* t, ApplyArgs* aa) {
     t->sc = P.d_sc;
     t->partials = P.d_partials;
     t->nparts = 0;
-    t->nblk = vec_blocks(P, (P.nb + 1) / 2);
+    t->threads = iter_threads(P);
+    t->nblk = vec_blocks(P, (P.nb + 1) / 2, t->threads);
     t->inv_nb = 1.0 / (double)P.nb;
     t->nb = P.nb;
     t->z = P.d_z;
@@ -590,14 +577,18 @@ cudaError_t iteration_args(Problem& P, IterArgs* t, ApplyArgs* aa) {
     t->w = P.d_w[(k + 1) % 2];
     t->x = P.d_x;
     t->tickets = reinterpret_cast<unsigned int*>(P.d_red + kTicketSlot);
+    if (fast_apply_supported(P, P.precision, aa->src_kind, aa->dst_kind, aa->stage)) {
+        aa->alpha_sc = P.d_sc;
+        aa->alpha_ticket = t->tickets + 2;
+    }
     t->hist = P.d_hist;
     return cudaSuccess;
 }
 
-cudaError_t group_iteration_tail(cudaStream_t s, const IterArgs* d_tab, int members, int max_blocks) {
-    FP_LAUNCHED(); k_alpha_g<<<members, 512, 0, s>>>(d_tab);
-    FP_LAUNCHED(); k_zupd_g<<<dim3(max_blocks, members), kVecThreads, 0, s>>>(d_tab);
-    FP_LAUNCHED(); k_vwupd_g<<<dim3(max_blocks, members), kVecThreads, 0, s>>>(d_tab);
+cudaError_t group_iteration_tail(cudaStream_t s, const IterArgs* d_tab, int members, int max_blocks,
+                                 int threads) {
+    launch_pdl(k_zupd_g, dim3(max_blocks, members), threads, 0, s, d_tab);
+    launch_pdl(k_vwupd_g, dim3(max_blocks, members), threads, 0, s, d_tab);
     return cudaGetLastError();
 }
 
@@ -608,12 +599,12 @@ cudaError_t minres_iteration(Problem& P) {
     int nparts = 0;
     cudaError_t e = launch_apply(P, a, &nparts);
     if (e != cudaSuccess) return e;
-    FP_LAUNCHED(); k_alpha<<<1, 512, 0, P.stream>>>(t.sc, t.partials, nparts, t.inv_nb);
+    if (!a.alpha_sc) launch_pdl(k_alpha, 1, 512, 0, P.stream, t.sc, t.partials, nparts, t.inv_nb);
     // the last block of k_zupd runs the Givens step, the last block of
     // k_vwupd the end of the iteration (block-count tickets in d_red)
-    FP_LAUNCHED(); k_zupd<<<t.nblk, kVecThreads, 0, P.stream>>>(t.sc, t.z, t.v, t.v_old, t.nb, t.partials,
+    launch_pdl(k_zupd, t.nblk, t.threads, 0, P.stream, t.sc, t.z, t.v, t.v_old, t.nb, t.partials,
                                                                  t.tickets, t.hist);
-    FP_LAUNCHED(); k_vwupd<<<t.nblk, kVecThreads, 0, P.stream>>>(t.sc, t.z, t.v, t.v_new, t.w_prev, t.w, t.x,
+    launch_pdl(k_vwupd, t.nblk, t.threads, 0, P.stream, t.sc, t.z, t.v, t.v_new, t.w_prev, t.w, t.x,
                                                                   t.nb, t.partials, t.tickets + 1);
     return cudaGetLastError();
 }
@@ -627,8 +618,9 @@ namespace {
 // v = scale * (v - mean), mean = sums[c] * inv_nb (AoS components; two
 // voxels per thread as in k_sum3)
 template <bool SCALE>
-__global__ void k_sub_mean(double* __restrict__ v, long long nb, const double* __restrict__ sums,
+__global__ void k_sub_mean(double* v, long long nb, const double* sums,
                            double inv_nb, double scale) {
+    pdl_wait();
     const double mz[3] = {sums[0] * inv_nb, sums[1] * inv_nb, sums[2] * inv_nb};
     const long long npair = nb >> 1;
     double2* v2 = reinterpret_cast<double2*>(v);
@@ -651,8 +643,9 @@ __global__ void k_sub_mean(double* __restrict__ v, long long nb, const double* _
 }
 
 // sums over the support of a dense SoA field, per component
-__global__ void k_gather_sum(const double* __restrict__ u, long long n, const int* __restrict__ support,
+__global__ void k_gather_sum(const double* u, long long n, const int* support,
                              long long nb, double* partials) {
+    pdl_wait();
     __shared__ double red[4 * 32];
     double acc[4] = {0, 0, 0, 0};
     for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < nb;
@@ -669,7 +662,8 @@ __global__ void k_gather_sum(const double* __restrict__ u, long long n, const in
 }
 
 // u[c] += add[c] on a dense SoA field
-__global__ void k_add_const3(double* __restrict__ u, long long n, const double* __restrict__ add) {
+__global__ void k_add_const3(double* u, long long n, const double* add) {
+    pdl_wait();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < 3 * n;
          i += (long long)gridDim.x * blockDim.x) {
         u[i] += add[i / n];
@@ -677,10 +671,11 @@ __global__ void k_add_const3(double* __restrict__ u, long long n, const double* 
 }
 
 // f0 on a dense SoA field (src/bignonnet/BackgroundForce.cpp:14-60)
-__global__ void k_background_force(const uint8_t* __restrict__ mask, long long n,
-                                   const int* __restrict__ support, long long nb, double cf0,
+__global__ void k_background_force(const uint8_t* mask, long long n,
+                                   const int* support, long long nb, double cf0,
                                    double cf1, double cf2, double cs0, double cs1, double cs2,
-                                   double* __restrict__ f0) {
+                                   double* f0) {
+    pdl_wait();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (long long)gridDim.x * blockDim.x) {
         const bool fl = mask[i] != 0;
@@ -695,8 +690,9 @@ __global__ void k_background_force(const uint8_t* __restrict__ mask, long long n
     (void)cs2;
 }
 
-__global__ void k_background_force_support(const int* __restrict__ support, long long nb, long long n,
-                                           double cs0, double cs1, double cs2, double* __restrict__ f0) {
+__global__ void k_background_force_support(const int* support, long long nb, long long n,
+                                           double cs0, double cs1, double cs2, double* f0) {
+    pdl_wait();
     for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < nb;
          s += (long long)gridDim.x * blockDim.x) {
         const long long v = support[s];
@@ -709,8 +705,9 @@ __global__ void k_background_force_support(const int* __restrict__ support, long
 }  // namespace
 
 // sum of (b - ax)^2 over the compact vectors, [blocks][4] partials with the sum in slot 3
-__global__ void k_resnorm(const double* __restrict__ b, const double* __restrict__ ax, long long m,
+__global__ void k_resnorm(const double* b, const double* ax, long long m,
                           double* partials) {
+    pdl_wait();
     __shared__ double red[4 * 32];
     double acc[4] = {0, 0, 0, 0};
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < m;
@@ -727,54 +724,44 @@ __global__ void k_resnorm(const double* __restrict__ b, const double* __restrict
 cudaError_t launch_resnorm(Problem& P, const double* b, const double* ax, double* out4) {
     const long long m = 3 * P.nb;
     const int blocks = vec_blocks(P, m);
-    FP_LAUNCHED(); k_resnorm<<<blocks, kVecThreads, 0, P.stream>>>(b, ax, m, P.d_partials);
-    FP_LAUNCHED(); k_reduce4<<<1, 512, 0, P.stream>>>(P.d_partials, blocks, out4);
+    launch_pdl(k_resnorm, blocks, kVecThreads, 0, P.stream, b, ax, m, P.d_partials);
+    launch_pdl(k_reduce4, 1, 512, 0, P.stream, P.d_partials, blocks, out4);
     return cudaGetLastError();
-}
-
-static __global__ void k_axpby(double* __restrict__ out, double a, const double* __restrict__ x, double b,
-                        const double* __restrict__ y, long long m) {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < m;
-         i += (long long)gridDim.x * blockDim.x)
-        out[i] = a * x[i] + b * y[i];
 }
 
 cudaError_t launch_axpby(Problem& P, double* out, double a, const double* x, double b,
                          const double* y) {
     const long long m = 3 * P.nb;
-    FP_LAUNCHED(); k_axpby<<<vec_blocks(P, m), kVecThreads, 0, P.stream>>>(out, a, x, b, y, m);
+    launch_pdl(k_axpby, vec_blocks(P, m), kVecThreads, 0, P.stream, out, a, x, b, y, m);
     return cudaGetLastError();
 }
 
 cudaError_t launch_sub_mean(Problem& P, double* v, const double* sums, double scale) {
     const int blocks = vec_blocks(P, (P.nb + 1) / 2);
     const double inv_nb = P.nb > 0 ? 1.0 / (double)P.nb : 0.0;
-    FP_LAUNCHED();
-    if (scale == 1.0)
-        k_sub_mean<false><<<blocks, kVecThreads, 0, P.stream>>>(v, P.nb, sums, inv_nb, scale);
-    else
-        k_sub_mean<true><<<blocks, kVecThreads, 0, P.stream>>>(v, P.nb, sums, inv_nb, scale);
+    launch_pdl(scale == 1.0 ? k_sub_mean<false> : k_sub_mean<true>, blocks, kVecThreads, 0, P.stream, v, P.nb,
+               sums, inv_nb, scale);
     return cudaGetLastError();
 }
 
 cudaError_t launch_gather_sum(Problem& P, const double* u_dense, double* out4) {
     const int blocks = vec_blocks(P, P.nb);
-    FP_LAUNCHED(); k_gather_sum<<<blocks, kVecThreads, 0, P.stream>>>(u_dense, P.n, P.d_support, P.nb,
+    launch_pdl(k_gather_sum, blocks, kVecThreads, 0, P.stream, u_dense, P.n, P.d_support, P.nb,
                                                         P.d_partials);
-    FP_LAUNCHED(); k_reduce4<<<1, 512, 0, P.stream>>>(P.d_partials, blocks, out4);
+    launch_pdl(k_reduce4, 1, 512, 0, P.stream, P.d_partials, blocks, out4);
     return cudaGetLastError();
 }
 
 cudaError_t launch_add_const3(Problem& P, double* u_dense, const double* add3) {
-    FP_LAUNCHED(); k_add_const3<<<vec_blocks(P, 3 * P.n), kVecThreads, 0, P.stream>>>(u_dense, P.n, add3);
+    launch_pdl(k_add_const3, vec_blocks(P, 3 * P.n), kVecThreads, 0, P.stream, u_dense, P.n, add3);
     return cudaGetLastError();
 }
 
 cudaError_t launch_background_force(Problem& P, const double cf[3], const double cs[3],
                                     double* f0) {
-    FP_LAUNCHED(); k_background_force<<<vec_blocks(P, P.n), kVecThreads, 0, P.stream>>>(
+    launch_pdl(k_background_force, vec_blocks(P, P.n), kVecThreads, 0, P.stream, 
         P.d_mask, P.n, P.d_support, P.nb, cf[0], cf[1], cf[2], cs[0], cs[1], cs[2], f0);
-    FP_LAUNCHED(); k_background_force_support<<<vec_blocks(P, P.nb), kVecThreads, 0, P.stream>>>(
+    launch_pdl(k_background_force_support, vec_blocks(P, P.nb), kVecThreads, 0, P.stream, 
         P.d_support, P.nb, P.n, cs[0], cs[1], cs[2], f0);
     return cudaGetLastError();
 }
