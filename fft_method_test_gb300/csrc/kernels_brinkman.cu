@@ -44,6 +44,33 @@ struct BrGrid {
     int nrows;  // ny * nz
 };
 
+// Exact division by a divisor d known before the launch, in two FP64
+// operations (Brisebarre, Muller and Raina, "Accelerating correctly rounded
+// floating-point division when the divisor is known in advance", IEEE Trans.
+// Computers 53(8), 2004): with zh = RN(1/d), zl = RN(1/d - zh),
+//     q = RN(x zh + RN(x zl)).
+// The value before the last rounding is within 2^-104 (relative) of x/d.  For
+// d = D 2^e with D odd, x/d keeps a relative distance of at least 2^-54 / D
+// from every rounding boundary (a boundary would need x = (2m + 1) D 2^k with
+// 2m + 1 of 54 bits), so q is the correctly rounded quotient, the value of
+// x / d, for every D < 2^40: zh = 0 marks other divisors (and infinite ones),
+// which divide.  Zeros (their sign), tiny and huge x divide as well.
+// GB300's FP64 pipe (two operations per clock and SM) bounds these kernels:
+// an outer iteration at 128^3 2289 -> 1657 us (35 sweeps of eight FP64
+// operations per voxel need 1180 us at the measured 498 G operations/s), at 48^3
+// 230 -> 176 us.
+struct BrDivisor {
+    double d, zh, zl;
+};
+
+__device__ __forceinline__ double br_div(double x, const BrDivisor& v) {
+    // 2^-600 <= |x| < 2^600 from the exponent bits: with 2^-200 < |d| < 2^200
+    // neither product underflows
+    const unsigned int e = (unsigned int)__double2hiint(x) & 0x7fffffffu;
+    if (v.zh == 0.0 || e - 0x1a700000u >= 0x65700000u - 0x1a700000u) return x / v.d;
+    return __fma_rn(x, v.zh, __dmul_rn(x, v.zl));
+}
+
 // Voxel loop of the stencil kernels: CTAs stride over the ny*nz grid rows,
 // threads over x, so neighbour indices need no per-voxel integer division.
 #define BR_FOR_VOXELS(g, row, x)                                      \
@@ -69,29 +96,30 @@ __device__ __forceinline__ void nbrs(const BrGrid& g, int row, int x, long long&
 }
 
 // FluidBrinkman.cpp:313-369
-__global__ void k_br_momentum(BrGrid g, const BrState* st, const uint8_t* __restrict__ fluid,
-                              double fluid_mu, double penalty, double relax, double f0, double f1,
-                              double f2, const double* __restrict__ ux, const double* __restrict__ uy,
-                              const double* __restrict__ uz, const double* __restrict__ p,
-                              double* __restrict__ sx, double* __restrict__ sy,
-                              double* __restrict__ sz) {
+__global__ void k_br_momentum(BrGrid g, const BrState* st, const uint8_t* fluid,
+                              double fluid_mu, BrDivisor dfluid, BrDivisor dsolid, double relax, double f0,
+                              double f1, double f2, const double* ux, const double* uy,
+                              const double* uz, const double* p,
+                              double* sx, double* sy,
+                              double* sz) {
+    pdl_wait();
     if (st->done) return;
     BR_FOR_VOXELS(g, row, x) {
         long long id, xm, xp, ym, yp, zm, zp;
         nbrs(g, row, x, id, xm, xp, ym, yp, zm, zp);
         const bool fl = fluid[id] != 0;
         const double mu = fl ? fluid_mu : 1.0;
-        const double alpha = fl ? 0.0 : penalty;
         const double lapUx = ux[xm] + ux[xp] + ux[ym] + ux[yp] + ux[zm] + ux[zp];
         const double lapUy = uy[xm] + uy[xp] + uy[ym] + uy[yp] + uy[zm] + uy[zp];
         const double lapUz = uz[xm] + uz[xp] + uz[ym] + uz[yp] + uz[zm] + uz[zp];
         const double dpdx = 0.5 * (p[xp] - p[xm]);
         const double dpdy = 0.5 * (p[yp] - p[ym]);
         const double dpdz = 0.5 * (p[zp] - p[zm]);
-        const double denom = alpha + 6.0 * mu;
-        const double jx = (f0 - dpdx + mu * lapUx) / denom;
-        const double jy = (f1 - dpdy + mu * lapUy) / denom;
-        const double jz = (f2 - dpdz + mu * lapUz) / denom;
+        // alpha + 6 mu: alpha = 0 in the fluid, the penalty in the solid
+        const BrDivisor denom = fl ? dfluid : dsolid;
+        const double jx = br_div(f0 - dpdx + mu * lapUx, denom);
+        const double jy = br_div(f1 - dpdy + mu * lapUy, denom);
+        const double jz = br_div(f2 - dpdz + mu * lapUz, denom);
         sx[id] = relax * jx + (1.0 - relax) * ux[id];
         sy[id] = relax * jy + (1.0 - relax) * uy[id];
         sz[id] = relax * jz + (1.0 - relax) * uz[id];
@@ -99,9 +127,10 @@ __global__ void k_br_momentum(BrGrid g, const BrState* st, const uint8_t* __rest
 }
 
 // FluidBrinkman.cpp:371-400, with per-CTA partial sums of div^2
-__global__ void k_br_divergence(BrGrid g, const BrState* st, const double* __restrict__ sx,
-                                const double* __restrict__ sy, const double* __restrict__ sz,
-                                double* __restrict__ div, double* partials) {
+__global__ void k_br_divergence(BrGrid g, const BrState* st, const double* sx,
+                                const double* sy, const double* sz,
+                                double* div, double* partials) {
+    pdl_wait();
     if (st->done) return;
     __shared__ double red[32];
     double acc[1] = {0.0};
@@ -118,32 +147,35 @@ __global__ void k_br_divergence(BrGrid g, const BrState* st, const double* __res
 }
 
 // First sweep from phi = 0: (0 + ... + 0 - div) / 6
-__global__ void k_br_jacobi0(BrGrid g, const BrState* st, const double* __restrict__ div,
-                             double* __restrict__ phin) {
+__global__ void k_br_jacobi0(BrGrid g, const BrState* st, const double* div,
+                             BrDivisor six, double* phin) {
+    pdl_wait();
     if (st->done) return;
     for (long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x; id < g.n;
          id += (long long)gridDim.x * blockDim.x)
-        phin[id] = (0.0 - div[id]) / 6.0;
+        phin[id] = br_div(0.0 - div[id], six);
 }
 
 // FluidBrinkman.cpp:402-433
-__global__ void k_br_jacobi(BrGrid g, const BrState* st, const double* __restrict__ phi,
-                            const double* __restrict__ div, double* __restrict__ phin) {
+__global__ void k_br_jacobi(BrGrid g, const BrState* st, const double* phi,
+                            const double* div, BrDivisor six, double* phin) {
+    pdl_wait();
     if (st->done) return;
     BR_FOR_VOXELS(g, row, x) {
         long long id, xm, xp, ym, yp, zm, zp;
         nbrs(g, row, x, id, xm, xp, ym, yp, zm, zp);
         const double nb = phi[xm] + phi[xp] + phi[ym] + phi[yp] + phi[zm] + phi[zp];
-        phin[id] = (nb - div[id]) / 6.0;
+        phin[id] = br_div(nb - div[id], six);
     }
 }
 
 // FluidBrinkman.cpp:435-466
-__global__ void k_br_project(BrGrid g, const BrState* st, const double* __restrict__ phi,
-                             const double* __restrict__ sx, const double* __restrict__ sy,
-                             const double* __restrict__ sz, double* __restrict__ ux,
-                             double* __restrict__ uy, double* __restrict__ uz,
-                             double* __restrict__ p) {
+__global__ void k_br_project(BrGrid g, const BrState* st, const double* phi,
+                             const double* sx, const double* sy,
+                             const double* sz, double* ux,
+                             double* uy, double* uz,
+                             double* p) {
+    pdl_wait();
     if (st->done) return;
     BR_FOR_VOXELS(g, row, x) {
         long long id, xm, xp, ym, yp, zm, zp;
@@ -159,8 +191,9 @@ __global__ void k_br_project(BrGrid g, const BrState* st, const double* __restri
 }
 
 // FluidBrinkman.cpp:468-497: residual, finiteness, stop test, counter
-__global__ void k_br_check(BrState* st, const double* __restrict__ partials, int nparts, long long n,
+__global__ void k_br_check(BrState* st, const double* partials, int nparts, long long n,
                            double tol, int maxit) {
+    pdl_wait();
     if (st->done) return;
     __shared__ double red[32];
     double acc[1] = {0.0};
@@ -183,8 +216,9 @@ __global__ void k_br_check(BrState* st, const double* __restrict__ partials, int
     }
 }
 
-__global__ void k_br_sum3(BrGrid g, const double* __restrict__ ux, const double* __restrict__ uy,
-                          const double* __restrict__ uz, double* partials) {
+__global__ void k_br_sum3(BrGrid g, const double* ux, const double* uy,
+                          const double* uz, double* partials) {
+    pdl_wait();
     __shared__ double red[4 * 32];
     double acc[4] = {0, 0, 0, 0};
     for (long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x; id < g.n;
@@ -222,6 +256,19 @@ struct BrBuffers {
         cudaFree(st);
     }
 };
+
+// zh, zl of br_div, or zh = 0 where the two-operation quotient is not proven
+BrDivisor br_divisor(double d) {
+    BrDivisor v{d, 0.0, 0.0};
+    if (!std::isfinite(d) || !(std::fabs(d) > 1e-60 && std::fabs(d) < 1e60)) return v;
+    int e = 0;
+    uint64_t m = (uint64_t)std::ldexp(std::fabs(std::frexp(d, &e)), 53);  // 53-bit integer mantissa
+    while ((m & 1u) == 0) m >>= 1;
+    if (m >= (1ull << 40)) return v;
+    v.zh = 1.0 / d;
+    v.zl = std::fma(-v.zh, d, 1.0) / d;  // 1 - zh d is exact
+    return v;
+}
 
 thread_local std::string g_brinkman_error;
 
@@ -306,20 +353,22 @@ extern "C" int fp_brinkman_solve(int nx, int ny, int nz, const uint32_t* ids, ui
     std::optional<CaptureGuard> capture_guard;
     capture_guard.emplace();
     cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
-    FP_LAUNCHED(); k_br_momentum<<<blocks, threads, 0, s>>>(g, b.st, b.fluid, fluid_mu, solid_penalty, relaxation,
-                                             force[0], force[1], force[2], ux, uy, uz, p, sx, sy, sz);
-    FP_LAUNCHED(); k_br_divergence<<<blocks, threads, 0, s>>>(g, b.st, sx, sy, sz, div, b.partials);
-    FP_LAUNCHED(); k_br_jacobi0<<<blocks, threads, 0, s>>>(g, b.st, div, phin);
+    const BrDivisor dfluid = br_divisor(0.0 + 6.0 * fluid_mu), dsolid = br_divisor(solid_penalty + 6.0 * 1.0);
+    const BrDivisor six = br_divisor(6.0);
+    launch_pdl(k_br_momentum, blocks, threads, 0, s, g, b.st, b.fluid, fluid_mu, dfluid, dsolid, relaxation,
+               force[0], force[1], force[2], ux, uy, uz, p, sx, sy, sz);
+    launch_pdl(k_br_divergence, blocks, threads, 0, s, g, b.st, sx, sy, sz, div, b.partials);
+    launch_pdl(k_br_jacobi0, blocks, threads, 0, s, g, b.st, div, six, phin);
     double* a = phin;  // current phi after sweep 1
     double* c = phi;
     for (int k = 1; k < 35; ++k) {
-        FP_LAUNCHED(); k_br_jacobi<<<blocks, threads, 0, s>>>(g, b.st, a, div, c);
+        launch_pdl(k_br_jacobi, blocks, threads, 0, s, g, b.st, a, div, six, c);
         double* t = a;
         a = c;
         c = t;
     }
-    FP_LAUNCHED(); k_br_project<<<blocks, threads, 0, s>>>(g, b.st, a, sx, sy, sz, ux, uy, uz, p);
-    FP_LAUNCHED(); k_br_check<<<1, 256, 0, s>>>(b.st, b.partials, blocks, n, tolerance, max_iterations);
+    launch_pdl(k_br_project, blocks, threads, 0, s, g, b.st, a, sx, sy, sz, ux, uy, uz, p);
+    launch_pdl(k_br_check, 1, 256, 0, s, b.st, b.partials, blocks, n, tolerance, max_iterations);
     cudaError_t e = cudaStreamEndCapture(s, &graph);
     if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
     capture_guard.reset();

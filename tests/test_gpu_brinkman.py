@@ -56,6 +56,19 @@ def test_brinkman_matches_oracle(gpu_lib, restatement, shape, seed):
     assert r["iterations"] == ro["iterations"]
 
 
+# both sides of the division rule: divisors 6 mu and penalty + 6 with a short
+# odd part (two-operation quotient) and with a full mantissa (division)
+@pytest.mark.parametrize("mu,penalty", [(1.0, 1e8), (1.0, 1234.5678), (0.7, 1e8), (0.375, 0.1)])
+def test_brinkman_divisors_match_oracle(gpu_lib, restatement, mu, penalty):
+    mask = (np.random.default_rng(21).random((9, 6, 33)) >= 0.4).astype(np.uint8)
+    ids = G.to_ids(mask)
+    ro = restatement.brinkman(ids, 1, mu, penalty, 0.9, 1e-8, 12, (0.2, -1.0, 0.5), want_fields=True)
+    r = brinkman(ids, (0.2, -1.0, 0.5), fluid_mu=mu, solid_penalty=penalty, max_iterations=12,
+                 want_fields=True)
+    for f in ("ux", "uy", "uz", "p"):
+        assert rel_err(r[f].ravel(), ro[f]) < 1e-14, f
+
+
 def test_brinkman_permeability_and_convergence(gpu_lib, restatement):
     from fft_method_test_gb300.permeability import computePermeabilityTensor
 
