@@ -21,12 +21,15 @@
 // residual that carries the pressure-gradient part (f - A x unprojected)
 // loses accuracy once |P r| << |r|.  One iteration:
 //     Ap = A p (7-point stencil), pAp = p . Ap       k_bf_stencil
-//     g = rho / pAp                                   k_bf_after_stencil
+//     g = rho / pAp                                   its last block
 //     a^ = F(Ap)                                      forward R2C FFT (3 passes)
 //     r^ -= g P^ a^,  z^ = r^ / (alpha0 + mu lambda)  k_bf_spectral
-//     rho' = <r^, z^> / N, beta = rho' / rho          k_bf_after_spectral
+//     rho' = <r^, z^> / N, beta = rho' / rho          its last block
 //     z = F^-1(z^)                                    inverse C2R FFT (3 passes)
 //     x += g p,  p = z + beta p                       k_bf_update
+// A chunk of iterations is one CUDA graph of programmatic launches (nine
+// kernels per iteration): 196 -> 164 us per iteration at 48^3, 320 -> 291 at
+// 64^3; the six FP64 transforms bound it.
 // Stop: |r^| / |r^_0| <= tol.  At the end the projected residual is
 // recomputed from x; if the recurrence ran ahead of it, CG restarts from x.
 // Only a uniform viscosity is a symmetric problem: fluid viscosity 1, the
@@ -40,6 +43,7 @@
 
 #include "../../include/fftperm.h"
 #include "internal.h"
+#include "minres_device.cuh"
 
 namespace fp {
 
@@ -57,29 +61,102 @@ struct BfScalars {
     double tol;
     long long it;
     long long maxit;
-    int stop;       // set by the reductions; copied to done at the end of the iteration
+    int stop;       // set by the reductions; the next iteration's stencil copies it to done
     int done;       // skips every kernel of later iterations
     int breakdown;  // pAp <= 0 or a non-finite scalar
-    int pad;
+    unsigned int ticket[2];  // block counts of k_bf_stencil and k_bf_spectral, zero between launches
 };
 
 constexpr int kBfThreads = 256;
+constexpr int kBfChunk = 25;  // iterations between two looks at the stop flag
 
 struct BfGrid {
     int nx, ny, nz;
     long long n;
 };
 
+__device__ __forceinline__ bool bad(double v) { return !isfinite(v); }
+
+// Sums of the first NV columns of the [nparts][4] partial rows, by one whole
+// block of any size, in the order of a block of 256 threads (8 warps): the
+// sums do not depend on the row length that sets the block size.
+template <int NV>
+__device__ __forceinline__ void sum_parts(const double* partials, int nparts, double* scratch, double (&out)[NV]) {
+    const int lane = threadIdx.x & 31;
+    for (int w = threadIdx.x >> 5; w < 8; w += (int)(blockDim.x >> 5)) {
+        double acc[NV] = {};
+        for (int i = 32 * w + lane; i < nparts; i += 256)
+#pragma unroll
+            for (int j = 0; j < NV; ++j) acc[j] += __ldcg(partials + 4LL * i + j);
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            const double v = warp_sum(acc[j]);
+            if (lane == 0) scratch[32 * j + w] = v;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 32)
+#pragma unroll
+        for (int j = 0; j < NV; ++j) out[j] = warp_sum(lane < 8 ? scratch[32 * j + lane] : 0.0);
+}
+
+// g = rho / pAp from the partial sums, by one whole block
+__device__ void after_stencil(BfScalars* sc, const double* partials, int nparts, double* red) {
+    double o[1];
+    sum_parts<1>(partials, nparts, red, o);
+    if (threadIdx.x == 0) {
+        const double pap = o[0];
+        sc->pap = pap;
+        if (sc->stop) {  // the iteration before was the last
+            sc->done = 1;
+        } else if (!(pap > 0.0) || bad(pap) || bad(sc->rho)) {
+            sc->breakdown = 1;
+            sc->stop = 1;
+            sc->g = 0.0;
+        } else {
+            sc->g = sc->rho / pap;
+        }
+    }
+}
+
+// rho', |r^|, beta, the stop test, by one whole block.  restart: beta = 0, the
+// iteration count unchanged, and r0 set when it is not yet known.
+__device__ void after_spectral(BfScalars* sc, const double* partials, int nparts, double inv_n, bool restart,
+                               double* red) {
+    double o[2];
+    sum_parts<2>(partials, nparts, red, o);
+    if (threadIdx.x == 0) {
+        const double rho = o[0] * inv_n;
+        const double rn = sqrt(o[1] * inv_n);
+        if (restart) {
+            if (!(sc->r0 > 0.0)) sc->r0 = rn;
+            sc->beta = 0.0;
+        } else {
+            sc->beta = rho / sc->rho;
+            sc->it += 1;
+        }
+        sc->rho = rho;
+        sc->rel = sc->r0 > 0.0 ? rn / sc->r0 : 0.0;
+        if (bad(rho) || bad(sc->beta)) {
+            sc->breakdown = 1;
+            sc->stop = 1;
+        }
+        if (sc->rel <= sc->tol || sc->it >= sc->maxit) sc->stop = 1;
+    }
+}
+
 // Ap = (alpha + 6) p - sum_nbr p for the three components (mu = 1), and
-// per-block partial sums of p . Ap.
-__global__ void __launch_bounds__(kBfThreads) k_bf_stencil(BfGrid g, const BfScalars* sc,
-                                                           const uint8_t* __restrict__ fluid,
+// per-block partial sums of p . Ap; with STEP the last block forms g.
+template <bool STEP>
+__global__ void __launch_bounds__(kBfThreads) k_bf_stencil(BfGrid g, BfScalars* sc,
+                                                           const uint8_t* fluid,
                                                            double penalty,
-                                                           const double* __restrict__ p,
-                                                           double* __restrict__ ap, double* partials) {
+                                                           const double* p,
+                                                           double* ap, double* partials) {
+    pdl_wait();
     __shared__ double red[4 * 32];
     if (sc->done) return;
-    double acc[4] = {0, 0, 0, 0};
+    double acc[1] = {0.0};
     const long long n = g.n;
     const long long sxy = (long long)g.nx * g.ny;
     // CTAs stride over grid rows, threads over x: no per-voxel division
@@ -98,41 +175,21 @@ __global__ void __launch_bounds__(kBfThreads) k_bf_stencil(BfGrid g, const BfSca
         const long long zm = (long long)(z == 0 ? g.nz - 1 : z - 1) * sxy + col;
         const long long zp = (long long)(z == g.nz - 1 ? 0 : z + 1) * sxy + col;
         const double diag = (fluid[id] ? 0.0 : penalty) + 6.0;
+        double a[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             const double* pc = p + c * n;
             const double v = pc[id];
-            const double a = diag * v - (pc[xm] + pc[xp] + pc[ym] + pc[yp] + pc[zm] + pc[zp]);
-            ap[c * n + id] = a;
-            acc[0] += v * a;
+            a[c] = diag * v - (pc[xm] + pc[xp] + pc[ym] + pc[yp] + pc[zm] + pc[zp]);
+            acc[0] += v * a[c];
         }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) ap[c * n + id] = a[c];
     }
-    double o[4];
-    block_sum<4>(acc, red, o);
+    double o[1];
+    block_sum<1>(acc, red, o);
     if (threadIdx.x == 0) partials[4LL * blockIdx.x] = o[0];
-}
-
-__device__ __forceinline__ bool bad(double v) { return !isfinite(v); }
-
-// g = rho / pAp (deterministic single-block reduction)
-__global__ void k_bf_after_stencil(BfScalars* sc, const double* partials, int nparts) {
-    __shared__ double red[4 * 32];
-    if (sc->done) return;
-    double acc[4] = {0, 0, 0, 0};
-    for (int i = threadIdx.x; i < nparts; i += blockDim.x) acc[0] += partials[4LL * i];
-    double o[4];
-    block_sum<4>(acc, red, o);
-    if (threadIdx.x == 0) {
-        const double pap = o[0];
-        sc->pap = pap;
-        if (!(pap > 0.0) || bad(pap) || bad(sc->rho)) {
-            sc->breakdown = 1;
-            sc->stop = 1;
-            sc->g = 0.0;
-        } else {
-            sc->g = sc->rho / pap;
-        }
-    }
+    if (STEP && last_block(&sc->ticket[0], gridDim.x)) after_stencil(sc, partials, (int)gridDim.x, red);
 }
 
 struct BfSpecArgs {
@@ -150,17 +207,19 @@ struct BfSpecArgs {
     double2* rhat;       // projected residual
     double fhat0[3];     // F(f) at k = 0 (N f); zero elsewhere for a uniform force
     double* partials;
+    double inv_n;
 };
 
 // mode 0 (iteration): r^ -= g P^ a^;  mode 1 (restart): r^ = P^ (F(f) - a^).
 // Then z^ = r^ / (alpha0 + mu lambda) into spec; partials {<r^, z^>, |r^|^2}
 // with the Hermitian weights of the half spectrum.
 template <int MODE>
-__global__ void __launch_bounds__(kBfThreads) k_bf_spectral(BfSpecArgs a, const BfScalars* sc) {
+__global__ void __launch_bounds__(kBfThreads) k_bf_spectral(BfSpecArgs a, BfScalars* sc) {
+    pdl_wait();
     __shared__ double red[4 * 32];
     if (sc->done) return;
     const double g = MODE == 0 ? sc->g : 0.0;
-    double acc[4] = {0, 0, 0, 0};
+    double acc[2] = {0.0, 0.0};
     const bool even = (a.nx & 1) == 0;
     for (int row = blockIdx.x; row < (int)a.nrows; row += gridDim.x)
         for (int kx = threadIdx.x; kx < a.nxh; kx += blockDim.x) {
@@ -217,71 +276,38 @@ __global__ void __launch_bounds__(kBfThreads) k_bf_spectral(BfSpecArgs a, const 
         acc[0] += w * d * rr;
         acc[1] += w * rr;
     }
-    double o[4];
-    block_sum<4>(acc, red, o);
+    double o[2];
+    block_sum<2>(acc, red, o);
     if (threadIdx.x == 0) {
         a.partials[4LL * blockIdx.x] = o[0];
         a.partials[4LL * blockIdx.x + 1] = o[1];
     }
-}
-
-// rho', |r^|, beta, the stop test.  restart: beta = 0, the iteration count
-// unchanged, and r0 set when it is not yet known.
-__global__ void k_bf_after_spectral(BfScalars* sc, const double* partials, int nparts, double inv_n,
-                                    int restart) {
-    __shared__ double red[4 * 32];
-    if (sc->done) return;
-    double acc[4] = {0, 0, 0, 0};
-    for (int i = threadIdx.x; i < nparts; i += blockDim.x) {
-        acc[0] += partials[4LL * i];
-        acc[1] += partials[4LL * i + 1];
-    }
-    double o[4];
-    block_sum<4>(acc, red, o);
-    if (threadIdx.x == 0) {
-        const double rho = o[0] * inv_n;
-        const double rn = sqrt(o[1] * inv_n);
-        if (restart) {
-            if (!(sc->r0 > 0.0)) sc->r0 = rn;
-            sc->beta = 0.0;
-        } else {
-            sc->beta = rho / sc->rho;
-            sc->it += 1;
-        }
-        sc->rho = rho;
-        sc->rel = sc->r0 > 0.0 ? rn / sc->r0 : 0.0;
-        if (bad(rho) || bad(sc->beta)) {
-            sc->breakdown = 1;
-            sc->stop = 1;
-        }
-        if (sc->rel <= sc->tol || sc->it >= sc->maxit) sc->stop = 1;
-    }
+    if (last_block(&sc->ticket[1], gridDim.x))
+        after_spectral(sc, a.partials, (int)gridDim.x, a.inv_n, MODE == 1, red);
 }
 
 // x += g p; p = z + beta p   (restart: g = 0, beta = 0, so p = z)
 template <int RESTART>
 __global__ void __launch_bounds__(kBfThreads) k_bf_update(const BfScalars* sc, long long m,
-                                                          double* __restrict__ x,
-                                                          double* __restrict__ p,
-                                                          const double* __restrict__ z) {
+                                                          double* x,
+                                                          double* p,
+                                                          const double* z) {
+    pdl_wait();
     if (sc->done) return;
     const double g = RESTART ? 0.0 : sc->g;
     const double beta = RESTART ? 0.0 : sc->beta;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < m;
          i += (long long)gridDim.x * blockDim.x) {
-        const double pv = p[i];
-        if (!RESTART) x[i] += g * pv;
-        p[i] = RESTART ? z[i] : z[i] + beta * pv;
+        const double pv = p[i], zv = z[i], xv = RESTART ? 0.0 : x[i];
+        if (!RESTART) x[i] = xv + g * pv;
+        p[i] = RESTART ? zv : zv + beta * pv;
     }
-}
-
-__global__ void k_bf_end(BfScalars* sc) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) sc->done = sc->stop;
 }
 
 // p^ = -i s . (F(f) - a^) / |s|^2 into component 0 of spec, components 1, 2
 // zeroed (pressure gauge: zero on the s = 0 modes).
 __global__ void k_bf_pressure(BfSpecArgs a) {
+    pdl_wait();
     for (int row = blockIdx.x; row < (int)a.nrows; row += gridDim.x)
         for (int kx = threadIdx.x; kx < a.nxh; kx += blockDim.x) {
         const int ky = row % a.ny;
@@ -307,7 +333,8 @@ __global__ void k_bf_pressure(BfSpecArgs a) {
     }
 }
 
-__global__ void k_bf_sum3(long long n, const double* __restrict__ u, double* partials) {
+__global__ void k_bf_sum3(long long n, const double* u, double* partials) {
+    pdl_wait();
     __shared__ double red[4 * 32];
     double acc[4] = {0, 0, 0, 0};
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -345,10 +372,13 @@ struct BfSolver {
     uint8_t* fluid = nullptr;
     BfScalars* sc = nullptr;
     BfScalars* hsc = nullptr;
+    cudaGraphExec_t graph = nullptr;  // kBfChunk iterations
+    long long graph_kernels = 0;
     int blocks = 0;
     int tx = kBfThreads;  // threads of the x-walking kernels (grid rows)
     int tk = kBfThreads;  // threads of the kx-walking kernels (spectral rows)
     ~BfSolver() {
+        if (graph) cudaGraphExecDestroy(graph);
         DeviceMemGuard mem_guard;
         cudaFree(x);
         cudaFree(p);
@@ -439,6 +469,7 @@ BfSpecArgs spec_args(BfSolver& S, const double f[3], double alpha0, double mu) {
     a.rhat = S.rhat;
     for (int c = 0; c < 3; ++c) a.fhat0[c] = (double)P.n * f[c];
     a.partials = P.d_partials;
+    a.inv_n = 1.0 / (double)P.n;
     return a;
 }
 
@@ -468,43 +499,55 @@ cudaError_t fft_inverse_dense(Problem& P, double* dst, const int* skip) {
 cudaError_t bf_iteration(BfSolver& S, const BfSpecArgs& sa, const BfGrid& g, double penalty) {
     Problem& P = S.h->P;
     const int* skip = &S.sc->done;
-    FP_LAUNCHED();
-    k_bf_stencil<<<S.blocks, S.tx, 0, P.stream>>>(g, S.sc, S.fluid, penalty, S.p, S.w,
-                                                         P.d_partials);
-    FP_LAUNCHED();
-    k_bf_after_stencil<<<1, 256, 0, P.stream>>>(S.sc, P.d_partials, S.blocks);
+    launch_pdl(k_bf_stencil<true>, S.blocks, S.tx, 0, P.stream, g, S.sc, S.fluid, penalty, S.p, S.w, P.d_partials);
     cudaError_t e = fft_forward_dense(P, S.w, skip);
     if (e != cudaSuccess) return e;
-    FP_LAUNCHED();
-    k_bf_spectral<0><<<S.blocks, S.tk, 0, P.stream>>>(sa, S.sc);
-    FP_LAUNCHED();
-    k_bf_after_spectral<<<1, 256, 0, P.stream>>>(S.sc, P.d_partials, S.blocks, 1.0 / (double)P.n, 0);
+    launch_pdl(k_bf_spectral<0>, S.blocks, S.tk, 0, P.stream, sa, S.sc);
     e = fft_inverse_dense(P, S.w, skip);
     if (e != cudaSuccess) return e;
-    FP_LAUNCHED();
-    k_bf_update<0><<<S.blocks, kBfThreads, 0, P.stream>>>(S.sc, 3 * P.n, S.x, S.p, S.w);
-    FP_LAUNCHED();
-    k_bf_end<<<1, 32, 0, P.stream>>>(S.sc);
+    launch_pdl(k_bf_update<0>, S.blocks, kBfThreads, 0, P.stream, S.sc, 3 * P.n, S.x, S.p, S.w);
     return cudaGetLastError();
+}
+
+// Queue a chunk of kBfChunk iterations: captured once per solver (an iteration
+// depends on neither the force nor the load case) and replayed.
+cudaError_t bf_chunk(BfSolver& S, const BfSpecArgs& sa, const BfGrid& g, double penalty) {
+    Problem& P = S.h->P;
+    if (!S.graph) {
+        CaptureGuard capture_guard;
+        const long long l0 = g_thread_launches;
+        cudaError_t e = cudaStreamBeginCapture(P.stream, cudaStreamCaptureModeThreadLocal);
+        if (e != cudaSuccess) return e;
+        cudaError_t le = cudaSuccess;
+        for (int i = 0; i < kBfChunk && le == cudaSuccess; ++i) le = bf_iteration(S, sa, g, penalty);
+        cudaGraph_t graph = nullptr;
+        e = cudaStreamEndCapture(P.stream, &graph);
+        S.graph_kernels = g_thread_launches - l0;
+        g_kernel_launches.fetch_sub(S.graph_kernels, std::memory_order_relaxed);  // nothing ran yet
+        if (e == cudaSuccess) e = le;
+        if (e == cudaSuccess) e = cudaGraphInstantiate(&S.graph, graph, 0);
+        if (graph) cudaGraphDestroy(graph);
+        if (e != cudaSuccess) {
+            S.graph = nullptr;
+            return e;
+        }
+    }
+    const cudaError_t e = cudaGraphLaunch(S.graph, P.stream);
+    if (e == cudaSuccess) g_kernel_launches.fetch_add(S.graph_kernels, std::memory_order_relaxed);
+    return e;
 }
 
 // r^ = P^ F(f - A x), z^ = M r^, p = z; sets rho, rel (and r0 when unset).
 // Leaves F(A x) overwritten; returns through hsc the new relative residual.
 cudaError_t bf_restart(BfSolver& S, const BfSpecArgs& sa, const BfGrid& g, double penalty) {
     Problem& P = S.h->P;
-    FP_LAUNCHED();
-    k_bf_stencil<<<S.blocks, S.tx, 0, P.stream>>>(g, S.sc, S.fluid, penalty, S.x, S.w,
-                                                         P.d_partials);
+    launch_pdl(k_bf_stencil<false>, S.blocks, S.tx, 0, P.stream, g, S.sc, S.fluid, penalty, S.x, S.w, P.d_partials);
     cudaError_t e = fft_forward_dense(P, S.w, nullptr);
     if (e != cudaSuccess) return e;
-    FP_LAUNCHED();
-    k_bf_spectral<1><<<S.blocks, S.tk, 0, P.stream>>>(sa, S.sc);
-    FP_LAUNCHED();
-    k_bf_after_spectral<<<1, 256, 0, P.stream>>>(S.sc, P.d_partials, S.blocks, 1.0 / (double)P.n, 1);
+    launch_pdl(k_bf_spectral<1>, S.blocks, S.tk, 0, P.stream, sa, S.sc);
     e = fft_inverse_dense(P, S.w, nullptr);
     if (e != cudaSuccess) return e;
-    FP_LAUNCHED();
-    k_bf_update<1><<<S.blocks, kBfThreads, 0, P.stream>>>(S.sc, 3 * P.n, S.x, S.p, S.w);
+    launch_pdl(k_bf_update<1>, S.blocks, kBfThreads, 0, P.stream, S.sc, 3 * P.n, S.x, S.p, S.w);
     return cudaGetLastError();
 }
 
@@ -541,7 +584,6 @@ int bf_solve(BfSolver& S, double penalty, double tol, long long maxit, const dou
     BF_CUDA(bf_restart(S, sa, g, penalty), "FFT Brinkman start");
     rc = bf_read(S);
     if (rc) return rc;
-    const int chunk = 25;
     const int max_restarts = 5;
     int restarts = 0;
     double true_rel = S.hsc->rel;
@@ -549,7 +591,7 @@ int bf_solve(BfSolver& S, double penalty, double tol, long long maxit, const dou
     while (!ok) {
         // iterate until the recurrence stops
         while (!S.hsc->stop) {
-            for (int i = 0; i < chunk; ++i) BF_CUDA(bf_iteration(S, sa, g, penalty), "FFT Brinkman iteration");
+            BF_CUDA(bf_chunk(S, sa, g, penalty), "FFT Brinkman iteration");
             rc = bf_read(S);
             if (rc) return rc;
         }
@@ -578,8 +620,7 @@ int bf_solve(BfSolver& S, double penalty, double tol, long long maxit, const dou
         return bf_fail(FP_ERR_NONFINITE, "FFT Brinkman: conjugate-gradient breakdown (non-finite or "
                                          "non-positive curvature)");
     // superficial velocity: mean of u over all voxels (FluidBrinkman.cpp:233-258)
-    FP_LAUNCHED();
-    k_bf_sum3<<<S.blocks, kBfThreads, 0, P.stream>>>(P.n, S.x, P.d_partials);
+    launch_pdl(k_bf_sum3, S.blocks, kBfThreads, 0, P.stream, P.n, S.x, P.d_partials);
     std::vector<double> part(4 * (size_t)S.blocks);
     BF_CUDA(cudaMemcpyAsync(part.data(), P.d_partials, sizeof(double) * part.size(),
                             cudaMemcpyDeviceToHost, P.stream),
@@ -599,12 +640,10 @@ int bf_solve(BfSolver& S, double penalty, double tol, long long maxit, const dou
         S.hsc->done = 0;
         rc = bf_write(S);
         if (rc) return rc;
-        FP_LAUNCHED();
-        k_bf_stencil<<<S.blocks, S.tx, 0, P.stream>>>(g, S.sc, S.fluid, penalty, S.x, S.w,
-                                                             P.d_partials);
+        launch_pdl(k_bf_stencil<false>, S.blocks, S.tx, 0, P.stream, g, S.sc, S.fluid, penalty, S.x, S.w,
+                   P.d_partials);
         BF_CUDA(fft_forward_dense(P, S.w, nullptr), "pressure FFT");
-        FP_LAUNCHED();
-        k_bf_pressure<<<S.blocks, S.tk, 0, P.stream>>>(sa);
+        launch_pdl(k_bf_pressure, S.blocks, S.tk, 0, P.stream, sa);
         BF_CUDA(fft_inverse_dense(P, S.w, nullptr), "pressure FFT");
         BF_CUDA(cudaMemcpyAsync(p_out, S.w, sizeof(double) * P.n, cudaMemcpyDeviceToHost, P.stream),
                 "copy");
