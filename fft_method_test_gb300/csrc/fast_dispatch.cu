@@ -10,18 +10,13 @@ namespace fp {
 namespace fast {
 
 // per-edge dispatch to the runners of fast_runners.cuh (instantiated in
-// fast32.cu, fast64.cu, fast32n.cu, fast64n.cu)
-#define FP_EDGE_SWITCH(n, CALL)                    \
-    switch (n) {                                   \
-        case 32: return CALL(32);                  \
-        case 48: return CALL(48);                  \
-        case 64: return CALL(64);                  \
-        case 80: return CALL(80);                  \
-        case 96: return CALL(96);                  \
-        case 128: return CALL(128);                \
-        case 160: return CALL(160);                \
-        case 256: return CALL(256);                \
-        default: break;                            \
+// the fast*.cu files)
+#define FP_EDGE_CASE(N) \
+    case N: return FP_CALL(N);
+#define FP_EDGE_SWITCH(n, CALL)          \
+    switch (n) {                         \
+        FP_FAST_EDGES(FP_EDGE_CASE)      \
+        default: break;                  \
     }
 
 template <typename T>
@@ -158,11 +153,11 @@ cudaError_t fast_plan(Problem& P, const ApplyArgs& aa, FastPlan<T>& pl) {
     pl.xgrid_i = std::min(pl.xgrid_i, kMaxPartials);
 
     // y passes: TX kx columns of one z plane and one component per CTA
-    constexpr int TX = fast::col_tx<T>();
+    const int TX = fast::y_tx_rt<T>(P.ny);
     const int ntx = (P.nxh + TX - 1) / TX;
     pl.ygrid = dim3(ntx, P.nz, 3);
     // z pass: persistent, TMA-fed, two pipeline stages per CTA
-    constexpr int TZ = fast::z_tx<T>();
+    const int TZ = fast::z_tx_rt<T>(P.nz);
     if (!fast_maps(P, sizeof(T) == 8, TZ, &pl.smap, &pl.gmap)) return cudaErrorNotSupported;
     // the tuning flag of the register-capped y/z kernels selects here the
     // single-stage z pass (three CTAs per SM instead of one two-stage CTA)

@@ -32,7 +32,7 @@ cudaError_t Passes<T, N>::xinv(const FastArgs& a, dim3 grid, int threads, size_t
 
 template <typename T, int N>
 cudaError_t Passes<T, N>::y(int dir, const FastArgs& a, dim3 grid, cudaStream_t s) {
-    constexpr int TX = col_tx<T>();
+    constexpr int TX = col_tx<T, N>();
     constexpr int NT = TX * Split<N>::TPL;
     if (a.group) {
         if (dir < 0)
@@ -51,7 +51,7 @@ cudaError_t Passes<T, N>::y(int dir, const FastArgs& a, dim3 grid, cudaStream_t 
 template <typename T, int N>
 cudaError_t Passes<T, N>::z(int stages, const CUtensorMap& spec_map, const CUtensorMap& green_map,
                             const FastArgs& a, dim3 grid, size_t smem, cudaStream_t s) {
-    constexpr int TX = z_tx<T>();
+    constexpr int TX = z_tx<T, N>();
     constexpr int NT = 3 * TX * Split<N>::TPL;
     if (a.group) {
         if (stages == 1)
@@ -69,14 +69,14 @@ cudaError_t Passes<T, N>::z(int stages, const CUtensorMap& spec_map, const CUten
 
 template <typename T, int N>
 cudaError_t Passes<T, N>::z_shared(const FastArgs& a, int grid, size_t smem, cudaStream_t s) {
-    constexpr int TX = z_tx<T>();
+    constexpr int TX = z_tx<T, N>();
     FP_RUN((k_fz_shared<T, N, TX>), grid, 3 * TX * Split<N>::TPL, smem, s, a);
     return cudaGetLastError();
 }
 
 template <typename T, int N>
 int Passes<T, N>::z_per_sm(int stages, size_t smem) {
-    constexpr int TX = z_tx<T>();
+    constexpr int TX = z_tx<T, N>();
     static std::atomic<unsigned long long> f1{0}, f2{0};
     int nb = 0;
     if (stages == 1) {

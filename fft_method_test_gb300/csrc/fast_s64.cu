@@ -1,0 +1,11 @@
+// fast_s64.cu -- the specialised apply passes in FP64 for the small edges of
+// fft_edges.cuh.
+#include "fast_runners.cuh"
+
+namespace fp {
+namespace fast {
+#define FP_INSTANCE(N, R1, R2, TPL) template struct Passes<double, N>;
+FP_EDGES_SMALL(FP_INSTANCE)
+#undef FP_INSTANCE
+}  // namespace fast
+}  // namespace fp

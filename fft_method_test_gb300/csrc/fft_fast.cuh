@@ -37,6 +37,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "fft_edges.cuh"
 #include "fft_engine.cuh"
 #include "internal.h"
 #include "minres_device.cuh"
@@ -45,8 +46,9 @@
 namespace fp {
 namespace fast {
 
-// N = R1 * R2 with R1 >= R2; TPL threads per line (TPL divides R1 and R2:
-// R2 for the powers of two, 4 for the edges with a factor 3 or 5).
+// N = R1 * R2; TPL threads per line.  For these eight edges TPL divides R1 and
+// R2 (R2 for the powers of two, 4 for the edges with a factor 3 or 5);
+// fft_edges.cuh lists the others.
 template <int N>
 struct Split;
 template <>
@@ -82,17 +84,58 @@ struct Split<256> {
     static constexpr int R1 = 16, R2 = 16, TPL = 16;
 };
 
+#define FP_SPLIT(N, A, B, T)                               \
+    template <>                                            \
+    struct Split<N> {                                      \
+        static constexpr int R1 = A, R2 = B, TPL = T;      \
+        static_assert(A * B == N && 32 % T == 0, "split"); \
+    };
+FP_EDGES_SMALL(FP_SPLIT)
+FP_EDGES_MIDDLE(FP_SPLIT)
+FP_EDGES_LARGE(FP_SPLIT)
+#undef FP_SPLIT
+
 // ---- small DFTs in natural order -------------------------------------------
 
 template <int P, int Q, int S, typename T2>
 __device__ __forceinline__ void dft_pfa(T2 (&v)[P * Q]);
 
+// DFT9 as 3 x 3: n = 3 n1 + n2, k = k1 + 3 k2, twiddles W9^(n2 k1).
+template <int S, typename T2>
+__device__ __forceinline__ void dft9(T2 (&v)[9]) {
+    using T = decltype(T2::x);
+    const T c1 = (T)0.76604444311897803520, s1 = (T)0.64278760968653932632;   // 2 pi / 9
+    const T c2 = (T)0.17364817766693034885, s2 = (T)0.98480775301220805937;   // 4 pi / 9
+    const T c4 = (T)-0.93969262078590838405, s4 = (T)0.34202014332566873304;  // 8 pi / 9
+#pragma unroll
+    for (int n2 = 0; n2 < 3; ++n2) dft3<S>(v[n2], v[3 + n2], v[6 + n2]);  // v[3 k1 + n2]
+    v[4] = mul_const<S>(v[4], c1, s1);
+    v[5] = mul_const<S>(v[5], c2, s2);
+    v[7] = mul_const<S>(v[7], c2, s2);
+    v[8] = mul_const<S>(v[8], c4, s4);
+#pragma unroll
+    for (int k1 = 0; k1 < 3; ++k1) dft3<S>(v[3 * k1], v[3 * k1 + 1], v[3 * k1 + 2]);  // X[k1 + 3 k2]
+    const T2 t[9] = {v[0], v[3], v[6], v[1], v[4], v[7], v[2], v[5], v[8]};
+#pragma unroll
+    for (int k = 0; k < 9; ++k) v[k] = t[k];
+}
+
 // Natural-order DFT of R values (S = -1 forward, +1 backward) with the
-// radix kernels of fft_engine.cuh (2, 3, 4, 5, 8, 16); 12 = 4 x 3 and
-// 20 = 4 x 5 by the prime-factor algorithm.
+// radix kernels of fft_engine.cuh (2, 3, 4, 5, 8, 16) and dft9; 6, 10, 12, 15,
+// 18 and 20 by the prime-factor algorithm.
 template <int R, int S, typename T2>
 __device__ __forceinline__ void dft_nat(T2 (&v)[R]) {
-    if constexpr (R == 12) {
+    if constexpr (R == 6) {
+        dft_pfa<2, 3, S>(v);
+    } else if constexpr (R == 9) {
+        dft9<S>(v);
+    } else if constexpr (R == 10) {
+        dft_pfa<2, 5, S>(v);
+    } else if constexpr (R == 15) {
+        dft_pfa<3, 5, S>(v);
+    } else if constexpr (R == 18) {
+        dft_pfa<2, 9, S>(v);
+    } else if constexpr (R == 12) {
         dft_pfa<4, 3, S>(v);
     } else if constexpr (R == 20) {
         dft_pfa<4, 5, S>(v);
@@ -151,7 +194,7 @@ __device__ __forceinline__ T2 twiddle(const T2* __restrict__ tw, int k, int a) {
 // either direction (RB = R2 forward, R1 inverse).
 template <int N>
 __host__ __device__ constexpr int line_span() {
-    return N + Split<N>::R1;
+    return N + (Split<N>::R1 > Split<N>::R2 ? Split<N>::R1 : Split<N>::R2);
 }
 
 // Column passes (thread = column + TX * (owner + TPL * comp)): one
@@ -208,7 +251,17 @@ __device__ __forceinline__ CtaBarrier make_group_barrier<CtaBarrier>(int, int) {
 
 // ---- four-step stages --------------------------------------------------------
 
-// Stage A for owners a = t + TPL*j (j < RB/TPL): loads RA values through
+// owners of a thread among R; with TPL not dividing R the last may be idle
+template <int R, int TPL>
+__host__ __device__ constexpr int owners() {
+    return (R + TPL - 1) / TPL;
+}
+template <int R, int TPL>
+__device__ __forceinline__ bool owned(int k) {
+    return R % TPL == 0 || k < R;
+}
+
+// Stage A for owners a = t + TPL*j (a < RB): loads RA values through
 // load(pos) (pos = RB*i + a), DFT-RA, twiddle W_N^(S a k), stores Y[k][a] at
 // line[k*(RB+1) + a].  With SYNC, bar() runs between the loads and the
 // stores (the loads read the same lines).
@@ -216,18 +269,20 @@ template <int RA, int RB, int S, int TPL, bool SYNC, typename T2, class Load,
           class Bar = CtaBarrier>
 __device__ __forceinline__ void stage_a(T2* line, int t, bool active, const T2* __restrict__ tw,
                                         Load& load, Bar bar = Bar{}) {
-    static_assert(RB % TPL == 0, "owners per thread");
-    constexpr int J = RB / TPL;
+    constexpr int J = owners<RB, TPL>();
     T2 v[J][RA];
 #pragma unroll
-    for (int j = 0; j < J; ++j)
+    for (int j = 0; j < J; ++j) {
+        const bool on = active && owned<RB, TPL>(t + TPL * j);
 #pragma unroll
-        for (int i = 0; i < RA; ++i) v[j][i] = active ? load(RB * i + t + TPL * j) : T2{};
+        for (int i = 0; i < RA; ++i) v[j][i] = on ? load(RB * i + t + TPL * j) : T2{};
+    }
     if (SYNC) bar();
     if (active) {
 #pragma unroll
         for (int j = 0; j < J; ++j) {
             const int a = t + TPL * j;
+            if (!owned<RB, TPL>(a)) continue;
             dft_nat<RA, S>(v[j]);
 #pragma unroll
             for (int k = 0; k < RA; ++k) {
@@ -239,26 +294,27 @@ __device__ __forceinline__ void stage_a(T2* line, int t, bool active, const T2* 
     }
 }
 
-// Stage B for owners k = t + TPL*j (j < RA/TPL): loads Y[k][a] (a < RB),
+// Stage B for owners k = t + TPL*j (k < RA): loads Y[k][a] (a < RB),
 // DFT-RB, hands X[k + RA*m] to store(pos, value).  With SYNC, bar() runs
 // between the loads and the stores.
 template <int RA, int RB, int S, int TPL, bool SYNC, typename T2, class Store,
           class Bar = CtaBarrier>
 __device__ __forceinline__ void stage_b(const T2* line, int t, bool active, Store& store,
                                         Bar bar = Bar{}) {
-    static_assert(RA % TPL == 0, "owners per thread");
-    constexpr int J = RA / TPL;
+    constexpr int J = owners<RA, TPL>();
     T2 u[J][RB];
 #pragma unroll
-    for (int j = 0; j < J; ++j)
+    for (int j = 0; j < J; ++j) {
+        const bool on = active && owned<RA, TPL>(t + TPL * j);
 #pragma unroll
-        for (int a = 0; a < RB; ++a)
-            u[j][a] = active ? line[(t + TPL * j) * (RB + 1) + a] : T2{};
+        for (int a = 0; a < RB; ++a) u[j][a] = on ? line[(t + TPL * j) * (RB + 1) + a] : T2{};
+    }
     if (SYNC) bar();
     if (active) {
 #pragma unroll
         for (int j = 0; j < J; ++j) {
             const int k = t + TPL * j;
+            if (!owned<RA, TPL>(k)) continue;
             dft_nat<RB, S>(u[j]);
 #pragma unroll
             for (int m = 0; m < RB; ++m) store(k + RA * m, u[j][m]);
@@ -382,6 +438,13 @@ __host__ __device__ constexpr int x_threads(int rows) {
 // [J-1-j][R2-1-m] of thread (TPL - t) % TPL, except for t = 0, whose mirror
 // images are its own registers: the two Hermitian halves meet through warp
 // shuffles, without shared memory.
+
+// That needs whole owners (TPL divides R1) and an even R2; other splits write
+// the transformed line back and read the mirror images from shared memory.
+template <int N>
+__host__ __device__ constexpr bool mirrored() {
+    return Split<N>::R1 % Split<N>::TPL == 0 && Split<N>::R2 % 2 == 0;
+}
 
 // the value of `v` in the mirror thread
 template <int TPL>
@@ -526,15 +589,13 @@ __global__ void __launch_bounds__(384) k_fx_fwd(const __grid_constant__ FastArgs
         //    stage B leaves X in registers), half spectra to HBM
         const bool act = q < nqa;
         T2* my = lines + (act ? q : 0) * LD;
-        T2 z[R1 / TPL][R2];
-        {
-            auto ld_nat = [&](int pos) { return my[pos]; };
-            stage_a<R1, R2, -1, TPL, true>(my, t, act, tw, ld_nat, WarpBarrier{});
-            __syncwarp();
+        auto ld_nat = [&](int pos) { return my[pos]; };
+        stage_a<R1, R2, -1, TPL, true>(my, t, act, tw, ld_nat, WarpBarrier{});
+        __syncwarp();
+        if constexpr (mirrored<N>()) {
+            T2 z[R1 / TPL][R2];
             stage_b_regs<R1, R2, -1, TPL>(my, t, act, z);
-        }
-        if (sizeof(T) == 4 && tile + gridDim.x >= a.ntiles) pdl_trigger();
-        {
+            if (sizeof(T) == 4 && tile + gridDim.x >= a.ntiles) pdl_trigger();
             T2* pa = spec + ca * a.nh + (r0 + rla) * KT;
             T2* pb = spec + cb * a.nh + (r0 + rlb) * KT;
             const bool hasb = act && Lb < nreal;
@@ -544,6 +605,21 @@ __global__ void __launch_bounds__(384) k_fx_fwd(const __grid_constant__ FastArgs
                 if (hasb) pb[o] = B;
             };
             separate_lines<R1, R2, TPL>(z, t, st);
+        } else {
+            auto st_nat = [&](int pos, T2 v) { my[pos] = v; };
+            stage_b<R1, R2, -1, TPL, true>(my, t, act, st_nat, WarpBarrier{});
+            __syncthreads();
+            if (sizeof(T) == 4 && tile + gridDim.x >= a.ntiles) pdl_trigger();
+            constexpr int NH = N / 2 + 1;
+            for (int it = tid; it < nqa * NH; it += nthr) {
+                const int qq = it / NH;
+                const int k = it - qq * NH;
+                const T2 zk = lines[qq * LD + k], zn = lines[qq * LD + (k == 0 ? 0 : N - k)];
+                const int L = 2 * qq, rl = L / 3, M = L + 1, rm = M / 3;
+                const long long o = (k / KT) * a.kts + k % KT;
+                spec[(L - 3 * rl) * a.nh + (r0 + rl) * KT + o] = cmk<T2>(zk.x + zn.x, zk.y - zn.y);
+                if (M < nreal) spec[(M - 3 * rm) * a.nh + (r0 + rm) * KT + o] = cmk<T2>(zk.y + zn.y, zn.x - zk.x);
+            }
         }
         __syncthreads();  // the lines are zeroed by the next tile
     }
@@ -601,9 +677,21 @@ __global__ void __launch_bounds__(384) k_fx_inv(const __grid_constant__ FastArgs
                 A = act ? pa[o] : T2{};
                 B = hasb ? pb[o] : T2{};
             };
-            T2 z[R1 / TPL][R2];
-            join_lines<R1, R2, TPL>(z, t, ld);
-            stage_a_regs<R2, R1, +1, TPL>(my, t, act, tw, z);
+            if constexpr (mirrored<N>()) {
+                T2 z[R1 / TPL][R2];
+                join_lines<R1, R2, TPL>(z, t, ld);
+                stage_a_regs<R2, R1, +1, TPL>(my, t, act, tw, z);
+            } else {
+                // Z = A + iB, above N/2 from the mirror image (read again, from L1)
+                auto ld_herm = [&](int k) {
+                    const bool lo = 2 * k <= N;
+                    T2 A, B;
+                    ld(lo ? k : N - k, A, B);
+                    if (k == 0 || 2 * k == N) A.y = B.y = (T)0;
+                    return lo ? cmk<T2>(A.x - B.y, A.y + B.x) : cmk<T2>(A.x + B.y, B.x - A.y);
+                };
+                stage_a<R2, R1, +1, TPL, false>(my, t, act, tw, ld_herm);
+            }
         }
         __syncwarp();
         {
@@ -694,6 +782,11 @@ __host__ __device__ constexpr int comp_stride() {
     return (int)(((size_t)TX * col_ld<N, T, TX>() * 2 * sizeof(T) + 127) / 128 * 128 /
                  (2 * sizeof(T)));
 }
+// Elements of one Green box [kz][TX], rounded up to whole 128 bytes as well.
+template <typename T, int N, int TX>
+__host__ __device__ constexpr int green_stride() {
+    return (int)(((size_t)TX * N * sizeof(T) + 127) / 128 * 128 / sizeof(T));
+}
 
 // Shared memory of one pipeline stage of the z pass: the spectral tile (per
 // component first raw [kz][TX] as the TMA box lands, then the padded lines
@@ -704,7 +797,7 @@ __host__ __device__ constexpr size_t z_green_offset() {
 }
 template <typename T, int N, int TX>
 __host__ __device__ constexpr size_t z_stage_bytes() {
-    return (z_green_offset<T, N, TX>() + (size_t)6 * N * TX * sizeof(T) + 127) & ~size_t(127);
+    return z_green_offset<T, N, TX>() + (size_t)6 * green_stride<T, N, TX>() * sizeof(T);
 }
 
 // Persistent CTAs walk the (kx tile, ky) tiles; thread = column + TX *
@@ -735,6 +828,7 @@ __global__ void __launch_bounds__(3 * TX * Split<N>::TPL, STAGES == 1 ? 3 : 1)
     constexpr int CS = comp_stride<T, N, TX>();
     constexpr size_t STAGE = z_stage_bytes<T, N, TX>();
     constexpr size_t GOFF = z_green_offset<T, N, TX>();
+    constexpr int GS = green_stride<T, N, TX>();
     constexpr uint32_t TILE_BYTES = (uint32_t)(3 * N * TX * sizeof(T2) + 6 * N * TX * sizeof(T));
     extern __shared__ __align__(128) unsigned char smem_raw[];
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw);
@@ -768,7 +862,7 @@ __global__ void __launch_bounds__(3 * TX * Split<N>::TPL, STAGES == 1 ? 3 : 1)
             tma_load_4d(base + (size_t)cc * CS * sizeof(T2), smap, 2 * ((ky << a.ktl) + (k0 & ((1 << a.ktl) - 1))), 0,
                         k0 >> a.ktl, cc, &bars[st]);
         for (int gc = 0; gc < 6; ++gc)
-            tma_load_4d(base + GOFF + (size_t)gc * N * TX * sizeof(T), gmap, k0, ky, 0, gc, &bars[st]);
+            tma_load_4d(base + GOFF + (size_t)gc * GS * sizeof(T), gmap, k0, ky, 0, gc, &bars[st]);
     };
 
     long long tile = blockIdx.x;
@@ -818,9 +912,9 @@ __global__ void __launch_bounds__(3 * TX * Split<N>::TPL, STAGES == 1 ? 3 : 1)
             const int g2 = comp == 0 ? 2 : (comp == 1 ? 4 : 5);
             auto ld_green = [&](int pos) {
                 const T2 X = lx[pos], Y = ly[pos], Z = lz[pos];
-                const T a0 = gsm[((size_t)g0 * N + pos) * TX + c];
-                const T a1 = gsm[((size_t)g1 * N + pos) * TX + c];
-                const T a2 = gsm[((size_t)g2 * N + pos) * TX + c];
+                const T a0 = gsm[g0 * GS + pos * TX + c];
+                const T a1 = gsm[g1 * GS + pos * TX + c];
+                const T a2 = gsm[g2 * GS + pos * TX + c];
                 return cmk<T2>(a0 * X.x + a1 * Y.x + a2 * Z.x, a0 * X.y + a1 * Y.y + a2 * Z.y);
             };
             stage_a<R2, R1, +1, TPL, true>(my, t, act, tw, ld_green);  // CTA barrier
@@ -862,7 +956,8 @@ __global__ void __launch_bounds__(3 * TX * Split<N>::TPL, sizeof(T) == 4 ? 2 : 1
     constexpr int LD = col_ld<N, T, TX>();
     constexpr int CS = comp_stride<T, N, TX>();
     constexpr size_t SPEC = z_green_offset<T, N, TX>();  // one spectral stage (128-byte multiple)
-    constexpr size_t GREEN = ((size_t)6 * N * TX * sizeof(T) + 127) & ~size_t(127);
+    constexpr int GS = green_stride<T, N, TX>();
+    constexpr size_t GREEN = (size_t)6 * GS * sizeof(T);
     constexpr uint32_t SPEC_BYTES = (uint32_t)(3 * N * TX * sizeof(T2));
     constexpr uint32_t GREEN_BYTES = (uint32_t)(6 * N * TX * sizeof(T));
     static_assert(128 + 2 * SPEC + 2 * GREEN <= 128 + 2 * z_stage_bytes<T, N, TX>(), "shared memory");
@@ -905,7 +1000,7 @@ __global__ void __launch_bounds__(3 * TX * Split<N>::TPL, sizeof(T) == 4 ? 2 : 1
         if (m == 0) {
             unsigned char* gb = green0 + ((i / G) & 1) * GREEN;
             for (int gc = 0; gc < 6; ++gc)
-                tma_load_4d(gb + (size_t)gc * N * TX * sizeof(T), &a0.group_maps[1], k0, ky, 0, gc,
+                tma_load_4d(gb + (size_t)gc * GS * sizeof(T), &a0.group_maps[1], k0, ky, 0, gc,
                             &bars[st]);
         }
     };
@@ -946,9 +1041,9 @@ __global__ void __launch_bounds__(3 * TX * Split<N>::TPL, sizeof(T) == 4 ? 2 : 1
             const int g2 = comp == 0 ? 2 : (comp == 1 ? 4 : 5);
             auto ld_green = [&](int pos) {
                 const T2 X = lx[pos], Y = ly[pos], Z = lz[pos];
-                const T a0g = gsm[((size_t)g0 * N + pos) * TX + c];
-                const T a1g = gsm[((size_t)g1 * N + pos) * TX + c];
-                const T a2g = gsm[((size_t)g2 * N + pos) * TX + c];
+                const T a0g = gsm[g0 * GS + pos * TX + c];
+                const T a1g = gsm[g1 * GS + pos * TX + c];
+                const T a2g = gsm[g2 * GS + pos * TX + c];
                 return cmk<T2>(a0g * X.x + a1g * Y.x + a2g * Z.x, a0g * X.y + a1g * Y.y + a2g * Z.y);
             };
             stage_a<R2, R1, +1, TPL, true>(my, t, act, tw, ld_green);  // CTA barrier
@@ -994,19 +1089,25 @@ cudaError_t fast_apply_group(Problem& P0, int precision, int members, const fast
 namespace fp {
 namespace fast {
 
-// kx columns per CTA of the y pass (64-byte row segments) and per tile of the
-// z pass (32-byte spectral rows, 16-byte FP32 Green rows: two CTAs per SM)
-template <typename T>
-constexpr int col_tx() {
-    return sizeof(T) == 4 ? 8 : 4;
+// kx columns per CTA of the y pass: 64-byte row segments, and at least a warp
+template <typename T, int N>
+__host__ __device__ constexpr int col_tx() {
+    constexpr int base = sizeof(T) == 4 ? 8 : 4, warp = 32 / Split<N>::TPL;
+    return base > warp ? base : warp;
 }
-template <typename T>
-constexpr int z_tx() {
+// kx columns per tile of the z pass
+template <typename T, int N>
+__host__ __device__ constexpr int z_tx() {
     return 4;
 }
 
 // grid edges with specialised kernels
-#define FP_FAST_EDGES(CALL) CALL(32) CALL(48) CALL(64) CALL(80) CALL(96) CALL(128) CALL(160) CALL(256)
+#define FP_FAST_EDGES(CALL)                                                                      \
+    CALL(32) CALL(48) CALL(64) CALL(80) CALL(96) CALL(128) CALL(160) CALL(256)                  \
+    CALL(20) CALL(24) CALL(25) CALL(27) CALL(30) CALL(36) CALL(40) CALL(45) CALL(50) CALL(54)   \
+    CALL(60) CALL(72) CALL(75) CALL(81) CALL(90) CALL(100) CALL(108) CALL(120)                  \
+    CALL(135) CALL(144) CALL(150) CALL(162) CALL(180) CALL(192) CALL(200) CALL(216) CALL(225)   \
+    CALL(240)
 
 inline bool edge_supported(int n) {
 #define FP_CASE(N) if (n == N) return true;
@@ -1043,6 +1144,13 @@ inline long long spec_elems(int nx, int ny, int nz) {
     return ((long long)((nx / 2 + 1 + (1 << l) - 1) >> l) << l) * ny * nz;
 }
 
+inline int x_tpl(int n) {
+#define FP_CASE(N) if (n == N) return Split<N>::TPL;
+    FP_FAST_EDGES(FP_CASE)
+#undef FP_CASE
+    return 0;
+}
+
 // grid rows per tile of the x passes: about 192 threads per CTA, 96 where
 // the lines are long and served by 4 threads (shared memory)
 inline int x_rows_for(int n) {
@@ -1054,14 +1162,11 @@ inline int x_rows_for(int n) {
         case 96: return 16;
         case 128: return 16;
         case 160: return 16;
-        default: return 8;
+        case 256: return 8;
+        default: break;
     }
-}
-inline int x_tpl(int n) {
-#define FP_CASE(N) if (n == N) return Split<N>::TPL;
-    FP_FAST_EDGES(FP_CASE)
-#undef FP_CASE
-    return 0;
+    const int tpl = x_tpl(n);  // about 192 threads, 96 where a line is long for its threads
+    return tpl >= 16 ? 8 : (tpl == 8 || n > 60 ? 16 : 32);
 }
 template <typename T>
 int x_ld_rt(int n) {
@@ -1071,11 +1176,26 @@ int x_ld_rt(int n) {
     return 0;
 }
 
+// column tile widths of the y and z passes
+template <typename T>
+int y_tx_rt(int n) {
+#define FP_CASE(N) if (n == N) return col_tx<T, N>();
+    FP_FAST_EDGES(FP_CASE)
+#undef FP_CASE
+    return 0;
+}
+template <typename T>
+int z_tx_rt(int n) {
+#define FP_CASE(N) if (n == N) return z_tx<T, N>();
+    FP_FAST_EDGES(FP_CASE)
+#undef FP_CASE
+    return 0;
+}
+
 // dynamic shared memory of the z pass: mbarriers + its pipeline stages
 template <typename T>
 size_t z_smem_rt(int n, int stages) {
-    constexpr int TX = z_tx<T>();
-#define FP_CASE(N) if (n == N) return 128 + stages * z_stage_bytes<T, N, TX>();
+#define FP_CASE(N) if (n == N) return 128 + stages * z_stage_bytes<T, N, z_tx<T, N>()>();
     FP_FAST_EDGES(FP_CASE)
 #undef FP_CASE
     return 0;
@@ -1083,7 +1203,8 @@ size_t z_smem_rt(int n, int stages) {
 
 // Launch runners of one edge, defined in fast_runners.cuh and instantiated
 // per precision and edge group (fast32.cu, fast64.cu: powers of two;
-// fast32n.cu, fast64n.cu: 48, 80, 96, 160) so that they build in parallel.
+// fast32n.cu, fast64n.cu: 48, 80, 96, 160; fast_{s,m,l}{32,64}.cu: the edges of
+// fft_edges.cuh) so that they build in parallel.
 // A set a.group selects the group kernels; the grid then carries the member
 // index (grid.y for the x and z passes, grid.z = 3 x members for the y pass).
 template <typename T, int N>
