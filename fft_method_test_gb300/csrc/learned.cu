@@ -13,8 +13,9 @@
 //            (the forward kernel with sign -1 on the offsets and W
 //            transposed per tap)
 //   wgrad    dW[tap][o][i] = sum_v dy[v][o] x[v + off(tap)][i]
-//            (per tap a GEMM over voxels; per-warp partials reduced in a
-//            fixed order: deterministic)
+//            (per tap a GEMM over voxels, wgrad.cuh; k_wgrad below for output
+//            counts that are no multiple of 16 and unaligned tensors; partials
+//            reduced in a fixed order: deterministic)
 // Channel counts: inputs of a convolution a multiple of 16 (the MMA's k),
 // outputs a multiple of 8 (its n), at most 64.
 #include <cuda_bf16.h>
@@ -22,7 +23,10 @@
 #include <stdint.h>
 
 #include "../../include/fftperm.h"
+#include <cooperative_groups.h>
+
 #include "common.cuh"
+#include "wgrad.cuh"
 
 namespace fp {
 namespace {
@@ -230,6 +234,49 @@ __global__ void k_wgrad_reduce(const float* __restrict__ partial, long long nchu
     }
 }
 
+// db[o] = sum_v dy[v][o] by one cluster: a thread takes one 16-byte piece (eight
+// channels) of every (cluster threads / pieces)-th row, so the reads are
+// contiguous; sums over the block's threads, then over the cluster's blocks
+// through distributed shared memory, in a fixed order.  (One block per channel
+// with strided two-byte loads read every sector once per channel.)
+constexpr int kBgThreads = 1024;
+__global__ void __launch_bounds__(kBgThreads) k_bias_grad_cluster(const uint4* __restrict__ dy, long long total,
+                                                                  int pieces, float* db) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    __shared__ float red[kBgThreads * 8];
+    const int tid = threadIdx.x;
+    const int rank = (int)cl.block_rank(), size = (int)cl.num_blocks();
+    float acc[8] = {};
+    const long long m = total * pieces;
+#pragma unroll 4
+    for (long long i = (long long)rank * kBgThreads + tid; i < m; i += (long long)size * kBgThreads) {
+        const uint4 u = dy[i];
+        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            acc[2 * k] += __uint_as_float(w[k] << 16);
+            acc[2 * k + 1] += __uint_as_float(w[k] & 0xffff0000u);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) red[tid * 8 + k] = acc[k];
+    __syncthreads();
+    for (int h = kBgThreads / 2; h >= pieces; h >>= 1) {
+        if (tid < h)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) red[tid * 8 + k] += red[(tid + h) * 8 + k];
+        __syncthreads();
+    }
+    cl.sync();
+    if (rank == 0 && tid < pieces * 8) {
+        float s = 0.f;
+        for (int r = 0; r < size; ++r) s += cl.map_shared_rank(red, r)[tid];
+        db[tid] = s;
+    }
+    cl.sync();  // the blocks' shared memory outlives the reads
+}
+
 // db[o] = sum_v dy[v][o]   (one CTA per output channel, fixed order)
 __global__ void k_bias_grad(const __nv_bfloat16* __restrict__ dy, long long total, int cout, float* db) {
     __shared__ float red[256];
@@ -399,8 +446,13 @@ extern "C" int fp_nn_wgrad(int nx, int ny, int nz, int64_t total, int dilation, 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     auto dy = static_cast<const __nv_bfloat16*>(dy_bf16);
     auto x = static_cast<const __nv_bfloat16*>(x_bf16);
-    const dim3 grid((unsigned)nchunks, 27);
     const int co16 = (cout + 15) / 16 * 16;
+    const fp::WgradArgs wa{nx, ny, nz, g.n, g.total, dilation, dy, cout, x, cin, (long long)chunk, partial, dw};
+    const bool covered = (co16 == 16 || co16 == 32 || (co16 == 64 && cin >= 32)) &&
+                         (cin == 16 || cin == 32 || (cin == 64 && co16 >= 32));
+    if (covered && fp::wgrad_ring_ok(wa)) return fp::wgrad_ring(wa, s) == cudaSuccess ? FP_OK : FP_ERR_CUDA;
+    // other output counts and unaligned tensors
+    const dim3 grid((unsigned)nchunks, 27);
 #define FP_WG(C16, CI)                                                                  \
     do {                                                                                \
         FP_LAUNCHED();                                                                  \
@@ -423,6 +475,28 @@ extern "C" int fp_nn_wgrad(int nx, int ny, int nz, int64_t total, int dilation, 
 
 extern "C" int fp_nn_bias_grad(const void* dy_bf16, int64_t total, int cout, float* db, void* stream) {
     if (!dy_bf16 || !db || total <= 0 || cout <= 0) return FP_ERR_INVALID;
+    const int pieces = cout / 8;
+    if (cout % 8 == 0 && (pieces & (pieces - 1)) == 0 && pieces <= 128 &&
+        (reinterpret_cast<uintptr_t>(dy_bf16) & 15) == 0) {
+        // as many blocks as have four reads per thread to do, at most a portable cluster
+        int blocks = 8;
+        while (blocks > 1 && (long long)total * pieces < 4LL * fp::kBgThreads * blocks) blocks /= 2;
+        cudaLaunchAttribute attr{};
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = (unsigned)blocks;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)blocks);
+        cfg.blockDim = dim3(fp::kBgThreads);
+        cfg.stream = static_cast<cudaStream_t>(stream);
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        FP_LAUNCHED();
+        return cudaLaunchKernelEx(&cfg, fp::k_bias_grad_cluster, static_cast<const uint4*>(dy_bf16),
+                                  (long long)total, pieces, db) == cudaSuccess
+                   ? FP_OK
+                   : FP_ERR_CUDA;
+    }
     FP_LAUNCHED();
     fp::k_bias_grad<<<cout, 256, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const __nv_bfloat16*>(dy_bf16), (long long)total, cout, db);

@@ -13,6 +13,7 @@
 
 #include "../../include/fftperm.h"
 #include "common.cuh"
+#include "wgrad.cuh"
 
 namespace fp {
 namespace {
@@ -251,6 +252,10 @@ extern "C" int fp_nn_wgrad_cc(int nx, int ny, int nz, int64_t total, int dilatio
     const long long nchunks = (total + chunk - 1) / chunk;
     if (nchunks > 65535) return FP_ERR_INVALID;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const fp::WgradArgs wa{nx, ny, nz, n, (long long)total, dilation, static_cast<const __nv_bfloat16*>(dy_bf16),
+                           cout, static_cast<const __nv_bfloat16*>(x_bf16), cin, (long long)chunk, partial, dw};
+    if (fp::wgrad_ring_ok(wa)) return fp::wgrad_ring(wa, s) == cudaSuccess ? FP_OK : FP_ERR_CUDA;
+    // unaligned tensors
     const dim3 grid((unsigned)nchunks, 27, (unsigned)((cout / 16) * (cin / 16)));
     FP_LAUNCHED();
     fp::k_wgrad_cc<<<grid, 256, 0, s>>>(nx, ny, nz, n, (long long)total, dilation,
