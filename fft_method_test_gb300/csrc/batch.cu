@@ -85,6 +85,15 @@ int time_apply(Problem& P, int reps, double* ms) {
         a.dst = P.d_cout;
         a.src_kind = kSrcCompact;
         a.dst_kind = kDstCompact;
+        // with the reduction to alpha that MINRES has the inverse x pass do: its
+        // length depends on the tiling (many small x tiles make many partial
+        // rows for one small last block)
+        if (fast_apply_supported(P, P.precision, a.src_kind, a.dst_kind, a.stage)) {
+            cudaMemsetAsync(P.d_sc, 0, sizeof(MinresScalars), P.stream);
+            a.dot_with = P.d_x;
+            a.alpha_sc = P.d_sc;
+            a.alpha_ticket = reinterpret_cast<unsigned int*>(P.d_red + kTicketSlot) + 2;
+        }
     } else {
         if (!P.d_dense_in && cudaMallocAsync(reinterpret_cast<void**>(&P.d_dense_in),
                                              sizeof(double) * 3 * (size_t)P.n, P.stream) != cudaSuccess)
