@@ -423,6 +423,28 @@ __device__ __forceinline__ const double2* tw_of<double>(const FastArgs& a, int a
     return axis == 0 ? a.tw64x : (axis == 1 ? a.tw64y : a.tw64z);
 }
 
+// A group member's arguments are copied out of the table into shared memory,
+// where a single apply has them in the constant bank: kept in registers they
+// cost the inverse x pass 109 instead of 80 registers per thread and half its
+// warps (122 against 67 us per member at 256^3 FP32 under ncu), and through a
+// reference to the table they would be reloaded after every global store.
+template <bool GROUP>
+struct ArgSlot {
+    unsigned long long w[GROUP ? (sizeof(FastArgs) + 7) / 8 : 1];
+};
+template <bool GROUP>
+__device__ __forceinline__ const FastArgs& member_args(const FastArgs& a0, int member, ArgSlot<GROUP>& slot) {
+    if constexpr (GROUP) {
+        static_assert(sizeof(FastArgs) % 8 == 0 && alignof(FastArgs) <= 8, "copied by 8-byte words");
+        const unsigned long long* src = reinterpret_cast<const unsigned long long*>(a0.group + member);
+        for (int i = threadIdx.x; i < (int)(sizeof(FastArgs) / 8); i += blockDim.x) slot.w[i] = src[i];
+        __syncthreads();
+        return *reinterpret_cast<const FastArgs*>(slot.w);
+    } else {
+        return a0;
+    }
+}
+
 // threads of the x passes for `rows` grid rows per tile: 3*rows/2 complex
 // lines of TPL threads, rounded up to whole warps
 template <int N>
@@ -531,11 +553,9 @@ constexpr int kMaxXLines = 48;
 // it (DRAM at 33 %, 22 warps per SM).
 template <typename T, int N, bool GROUP>
 __global__ void __launch_bounds__(384) k_fx_fwd(const __grid_constant__ FastArgs a0) {
-    // a group member's arguments are copied out of the table once: read
-    // through a reference they would be reloaded after every global store
     pdl_wait();
-    const FastArgs ag = GROUP ? a0.group[blockIdx.y] : FastArgs{};
-    const FastArgs& a = GROUP ? ag : a0;
+    __shared__ ArgSlot<GROUP> slot;
+    const FastArgs& a = member_args<GROUP>(a0, blockIdx.y, slot);
     if (a.skip && *a.skip) return;
     using T2 = c_t<T>;
     constexpr int R1 = Split<N>::R1, R2 = Split<N>::R2, TPL = Split<N>::TPL;
@@ -637,8 +657,8 @@ __global__ void __launch_bounds__(384) k_fx_fwd(const __grid_constant__ FastArgs
 template <typename T, int N, bool GROUP>
 __global__ void __launch_bounds__(384) k_fx_inv(const __grid_constant__ FastArgs a0) {
     pdl_wait();
-    const FastArgs ag = GROUP ? a0.group[blockIdx.y] : FastArgs{};
-    const FastArgs& a = GROUP ? ag : a0;
+    __shared__ ArgSlot<GROUP> slot;
+    const FastArgs& a = member_args<GROUP>(a0, blockIdx.y, slot);
     if (a.skip && *a.skip) return;
     using T2 = c_t<T>;
     constexpr int R1 = Split<N>::R1, R2 = Split<N>::R2, TPL = Split<N>::TPL;
@@ -739,8 +759,8 @@ __global__ void __launch_bounds__(384) k_fx_inv(const __grid_constant__ FastArgs
 template <typename T, int N, int S, int TX, bool GROUP>
 __global__ void __launch_bounds__(TX * Split<N>::TPL) k_fcol_y(const __grid_constant__ FastArgs a0) {
     pdl_wait();
-    const FastArgs ag = GROUP ? a0.group[blockIdx.z / 3] : FastArgs{};
-    const FastArgs& a = GROUP ? ag : a0;
+    __shared__ ArgSlot<GROUP> slot;
+    const FastArgs& a = member_args<GROUP>(a0, blockIdx.z / 3, slot);
     const int comp = GROUP ? (int)(blockIdx.z % 3) : (int)blockIdx.z;
     if (a.skip && *a.skip) return;
     using T2 = c_t<T>;

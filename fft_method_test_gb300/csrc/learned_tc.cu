@@ -10,13 +10,15 @@
 // [27][cout][cin] (the data gradient passes the per-tap transposed weights
 // and sign -1), periodic wrap, FP32 accumulation.  Per tap the 128 shifted
 // input rows (A, 128 x cin) and the tap's weights (B, cout x cin) are
-// copied into one of two shared-memory buffers with cp.async, in the
+// copied into one of STAGES shared-memory buffers with cp.async, in the
 // canonical K-major layout without swizzle: 8 x 16-byte core matrices, the
 // two core matrices of a 16-channel chunk side by side (leading byte offset
 // 128), 8-row groups 256 bytes apart (stride byte offset).  One thread issues
 // cin/16 MMAs of 128 x cout x 16 per tap and commits them to the buffer's
-// mbarrier, so the 128 threads gather tap t + 1 while the tensor cores work
-// on tap t.  The epilogue reads the accumulator rows back with tcgen05.ld
+// mbarrier; the 128 threads meanwhile gather the rows of tap t + STAGES - 1, so
+// the latency of a gather is hidden by STAGES - 1 taps (waiting for each tap's
+// rows made the kernel 27 L2 latencies long: CONV_FIGURES).  A grid of few
+// voxels splits the output channels over blockIdx.y.  The epilogue reads the accumulator rows back with tcgen05.ld
 // (warp w owns TMEM lanes 32w..32w+31 = voxel rows), adds the bias, applies
 // ReLU and stores FP32 and/or BF16.
 //
@@ -55,6 +57,7 @@ struct TcConv {
     int dil, sign;
     const __nv_bfloat16* in;
     int cin;
+    int cout;  // all output channels (a CTA computes COUT of them)
     const __nv_bfloat16* w;
     const float* bias;
     int relu;
@@ -98,16 +101,18 @@ __device__ __forceinline__ uint32_t core_offset(int m, int q, int rows) {
     return (uint32_t)((q >> 1) * rows * 32 + ((m >> 3) * 2 + (q & 1)) * 128 + (m & 7) * 16);
 }
 
-template <int COUT>
+template <int COUT, int STAGES>
 __global__ void __launch_bounds__(kTcThreads) k_conv_tc(TcConv p) {
     constexpr int NCOLS = COUT < 32 ? 32 : COUT;  // TMEM columns (power of two, >= 32)
     extern __shared__ __align__(1024) unsigned char sm[];
     uint64_t* bars = reinterpret_cast<uint64_t*>(sm);
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + 16);
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + 64);
+    volatile int* failed = reinterpret_cast<volatile int*>(sm + 72);
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
     const int cin = p.cin;
     const int kc = cin / 16;
+    const int o0 = blockIdx.y * COUT;
     const uint32_t abytes = (uint32_t)kTcM * cin * 2;
     const uint32_t bbytes = (uint32_t)COUT * cin * 2;
     unsigned char* buf0 = sm + 1024;
@@ -122,16 +127,16 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_tc(TcConv p) {
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
-        mbar_init(&bars[0], 1);
-        mbar_init(&bars[1], 1);
+        for (int b = 0; b < STAGES; ++b) mbar_init(&bars[b], 1);
         fence_mbar_init();
+        *failed = 0;
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tslot;
 
-    // this thread's voxel (A row tid)
+    // this thread's voxel (A row tid) and its wrapped neighbours along each axis
     const long long v = (long long)blockIdx.x * kTcM + tid;
     const bool valid = v < p.total;
     const long long vv = valid ? v : 0;
@@ -142,25 +147,24 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_tc(TcConv p) {
     const int y = (int)(q0 % p.ny);
     const int z = (int)(q0 / p.ny);
     const int step = p.sign * p.dil;
+    auto wrap = [](int i, int n) {
+        i %= n;
+        return i < 0 ? i + n : i;
+    };
+    const int xm = wrap(x - step, p.nx), xp = wrap(x + step, p.nx);
+    const int ym = wrap(y - step, p.ny), yp = wrap(y + step, p.ny);
+    const int zm = wrap(z - step, p.nz), zp = wrap(z + step, p.nz);
+    const __nv_bfloat16* in = p.in + smp * p.n * cin;
 
-    bool ok = true;
-    int last = 0;
-    for (int tap = 0; tap < 27; ++tap) {
-        const int b = tap & 1;
-        // the MMAs of tap - 2 read this buffer
-        if (tap >= 2 && !tma_pipeline_wait<float2>(bars, tap - 2, b, true, &g_tc_err)) {
-            ok = false;
-            break;
-        }
+    auto issue = [&](int tap) {
+        const int b = tap % STAGES;
         // A: the shifted input row of this voxel
         {
-            const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-            int xx = (x + step * dx) % p.nx, yy = (y + step * dy) % p.ny, zz = (z + step * dz) % p.nz;
-            if (xx < 0) xx += p.nx;
-            if (yy < 0) yy += p.ny;
-            if (zz < 0) zz += p.nz;
-            const long long nb = smp * p.n + ((long long)zz * p.ny + yy) * p.nx + xx;
-            const __nv_bfloat16* src = p.in + nb * cin;
+            const int dz = tap / 9, dy = tap / 3 % 3, dx = tap % 3;
+            const int zz = dz == 0 ? zm : (dz == 1 ? z : zp);
+            const int yy = dy == 0 ? ym : (dy == 1 ? y : yp);
+            const int xx = dx == 0 ? xm : (dx == 1 ? x : xp);
+            const __nv_bfloat16* src = in + (((long long)zz * p.ny + yy) * p.nx + xx) * cin;
             unsigned char* a = abuf(b);
             for (int q = 0; q < cin / 8; ++q)
                 cp_async16_zfill(a + core_offset(tid, q, kTcM), src + q * 8, valid);
@@ -168,7 +172,7 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_tc(TcConv p) {
         // B: the tap's weights [cout][cin]
         {
             const int per = cin / 8;
-            const __nv_bfloat16* wt = p.w + (size_t)tap * COUT * cin;
+            const __nv_bfloat16* wt = p.w + ((size_t)tap * p.cout + o0) * cin;
             unsigned char* bm = bbuf(b);
             for (int i = tid; i < COUT * per; i += kTcThreads) {
                 const int co = i / per;
@@ -176,9 +180,24 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_tc(TcConv p) {
                 cp_async16_zfill(bm + core_offset(co, q, COUT), wt + (size_t)co * cin + q * 8, true);
             }
         }
-        asm volatile("cp.async.wait_all;" ::: "memory");
+    };
+
+    bool ok = true;
+#pragma unroll
+    for (int tap = 0; tap < STAGES - 1; ++tap) {
+        issue(tap);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    for (int tap = 0; tap < 27; ++tap) {
+        const int b = tap % STAGES;
+        // this thread's copies of the tap, then everybody's
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
         fence_proxy_async_smem();
         __syncthreads();
+        if (*failed) {
+            ok = false;
+            break;
+        }
         if (tid == 0) {
             tc_fence_after();
             const unsigned char* a = abuf(b);
@@ -201,10 +220,24 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_tc(TcConv p) {
                     smem_u32(&bars[b]))
                 : "memory");
         }
-        last = tap;
+        // tap + STAGES - 1 goes where the MMAs of tap - 1 read
+        const int nt = tap + STAGES - 1;
+        if (nt < 27) {
+            if (tap >= 1 &&
+                !mbar_wait_bounded(&bars[(tap - 1) % STAGES], (uint32_t)(((tap - 1) / STAGES) & 1)))
+                *failed = 1;  // every thread sees it after the next barrier
+            else
+                issue(nt);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     // the last commit covers every MMA issued before it
-    if (ok) ok = tma_pipeline_wait<float2>(bars, last, last & 1, false, &g_tc_err);
+    if (ok) ok = mbar_wait_bounded(&bars[26 % STAGES], (uint32_t)((26 / STAGES) & 1));
+    if (__syncthreads_or(!ok)) {
+        ok = false;
+        if (tid == 0) atomicExch(&g_tc_err, 1);
+    }
     tc_fence_after();
     if (ok) {
         // epilogue: TMEM lanes 32w..32w+31 are the rows of warp w
@@ -224,12 +257,12 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_tc(TcConv p) {
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
                 f[j] = __uint_as_float(rr[j]);
-                if (p.bias) f[j] += p.bias[c0 + j];
+                if (p.bias) f[j] += p.bias[o0 + c0 + j];
                 if (p.relu) f[j] = fmaxf(f[j], 0.f);
             }
             if (valid) {
                 if (p.out32) {
-                    float4* o = reinterpret_cast<float4*>(p.out32 + v * COUT + c0);
+                    float4* o = reinterpret_cast<float4*>(p.out32 + v * p.cout + o0 + c0);
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
                         o[j] = make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
@@ -242,7 +275,7 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_tc(TcConv p) {
                         const uint32_t hi = __bfloat16_as_ushort(__float2bfloat16(f[2 * j + 1]));
                         pk[j] = lo | (hi << 16);
                     }
-                    uint4* o = reinterpret_cast<uint4*>(p.out16 + v * COUT + c0);
+                    uint4* o = reinterpret_cast<uint4*>(p.out16 + v * p.cout + o0 + c0);
                     o[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
                     o[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
                 }
@@ -268,11 +301,11 @@ void ensure_smem_limit(K kern, std::atomic<unsigned long long>& done) {
     }
 }
 
-// shared memory of one CTA: barriers + two buffers, and at least the CTA's
+// shared memory of one CTA: barriers + its buffers, and at least the CTA's
 // share of the SM for its TMEM columns
-size_t tc_smem(int cin, int cout) {
-    const int ncols = cout < 32 ? 32 : cout;
-    const size_t need = 1024 + 2 * ((size_t)kTcM * cin * 2 + (size_t)cout * cin * 2);
+size_t tc_smem(int cin, int tile, int stages) {
+    const int ncols = tile < 32 ? 32 : tile;
+    const size_t need = 1024 + stages * ((size_t)kTcM * cin * 2 + (size_t)tile * cin * 2);
     const size_t share = (size_t)233472 * ncols / 512;
     return need > share ? need : share;
 }
@@ -288,28 +321,39 @@ extern "C" int fp_nn_conv_tc(int nx, int ny, int nz, int64_t total, int dilation
         return FP_ERR_INVALID;
     if (dilation < 1 || (sign != 1 && sign != -1)) return FP_ERR_INVALID;
     fp::TcConv p{nx, ny, nz, (long long)nx * ny * nz, (long long)total, dilation, sign,
-                 static_cast<const __nv_bfloat16*>(in_bf16), cin,
+                 static_cast<const __nv_bfloat16*>(in_bf16), cin, cout,
                  static_cast<const __nv_bfloat16*>(w_bf16), bias, relu, out_f32,
                  static_cast<__nv_bfloat16*>(out_bf16)};
     if (p.total % p.n) return FP_ERR_INVALID;
     const long long blocks = (p.total + fp::kTcM - 1) / fp::kTcM;
     if (blocks > 0x7fffffffLL) return FP_ERR_INVALID;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const size_t smem = fp::tc_smem(cin, cout);
+    if (cout != 16 && cout != 32 && cout != 64 && cout != 128) return FP_ERR_INVALID;
+    // Output channels per CTA: all of them (the gathered rows serve them all)
+    // while the voxels alone give two CTAs per SM; fewer voxels, as on the
+    // coarse levels, split the channels down to 32.
+    int tile = cout;
+    while (tile > 32 && blocks * (cout / tile) < 304) tile /= 2;
+    // Four buffers where several CTAs still fit an SM (48 KB), else three.
+    const int stages = fp::tc_smem(cin, tile, 4) <= 49152 ? 4 : 3;
+    const size_t smem = fp::tc_smem(cin, tile, stages);
     if (smem > 232448) return FP_ERR_INVALID;
-#define FP_TC_LAUNCH(C)                                                                           \
+#define FP_TC_LAUNCH(C, S)                                                                        \
     {                                                                                             \
         static std::atomic<unsigned long long> done_{0};                                          \
-        fp::ensure_smem_limit(fp::k_conv_tc<C>, done_);                                               \
+        fp::ensure_smem_limit(fp::k_conv_tc<C, S>, done_);                                        \
         FP_LAUNCHED();                                                                            \
-        fp::k_conv_tc<C><<<(unsigned)blocks, fp::kTcThreads, smem, s>>>(p);                       \
+        fp::k_conv_tc<C, S><<<dim3((unsigned)blocks, (unsigned)(cout / C)), fp::kTcThreads, smem, s>>>(p); \
     }
-    switch (cout) {
-        case 16: FP_TC_LAUNCH(16) break;
-        case 32: FP_TC_LAUNCH(32) break;
-        case 64: FP_TC_LAUNCH(64) break;
-        case 128: FP_TC_LAUNCH(128) break;
-        default: return FP_ERR_INVALID;
+    switch (tile * 10 + stages) {
+        case 163: FP_TC_LAUNCH(16, 3) break;
+        case 164: FP_TC_LAUNCH(16, 4) break;
+        case 323: FP_TC_LAUNCH(32, 3) break;
+        case 324: FP_TC_LAUNCH(32, 4) break;
+        case 643: FP_TC_LAUNCH(64, 3) break;
+        case 644: FP_TC_LAUNCH(64, 4) break;
+        case 1283: FP_TC_LAUNCH(128, 3) break;
+        default: FP_TC_LAUNCH(128, 4) break;
     }
 #undef FP_TC_LAUNCH
     return cudaGetLastError() == cudaSuccess ? FP_OK : FP_ERR_CUDA;
