@@ -480,7 +480,7 @@ extern "C" int fp_nn_bias_grad(const void* dy_bf16, int64_t total, int cout, flo
         (reinterpret_cast<uintptr_t>(dy_bf16) & 15) == 0) {
         // as many blocks as have four reads per thread to do, at most a cluster of 16
         // (four 64^3 cells with 16 channels: 81 us with 8 blocks and four reads in
-        // flight per thread, BG_FIGURES with 16 and eight)
+        // flight per thread, 45 with 16 and eight)
         static const bool wide = cudaFuncSetAttribute(fp::k_bias_grad_cluster,
                                                       cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
         int blocks = wide ? 16 : 8;

@@ -4,7 +4,8 @@
 // reference (its MinresSolver::solve takes an initial guess,
 // src/solver/MinresSolver.hpp:23, that nothing fills).
 //
-// Implicit GEMM, one CTA per 128 voxels (the MMA's M):
+// Implicit GEMM, one CTA per 128 voxels (the MMA's M), in two forms: k_conv_halo
+// below (dilation 1, up to 64 input channels) and, for the rest, k_conv_tc:
 //   y[v][o] = sum_tap sum_i x[v + sign*dil*off(tap)][i] W[tap][o][i]
 // Activations are channels-last BF16 [voxel][channel], weights BF16
 // [27][cout][cin] (the data gradient passes the per-tap transposed weights
@@ -16,8 +17,9 @@
 // 128), 8-row groups 256 bytes apart (stride byte offset).  One thread issues
 // cin/16 MMAs of 128 x cout x 16 per tap and commits them to the buffer's
 // mbarrier; the 128 threads meanwhile gather the rows of tap t + STAGES - 1, so
-// the latency of a gather is hidden by STAGES - 1 taps (waiting for each tap's
-// rows made the kernel 27 L2 latencies long: CONV_FIGURES).  A grid of few
+// the latency of a gather is hidden by STAGES - 1 taps (128 -> 128 channels on
+// four 8^3 cells: 101 us waiting for each tap's rows, 52 with this and the split
+// output channels).  A grid of few
 // voxels splits the output channels over blockIdx.y.  The epilogue reads the accumulator rows back with tcgen05.ld
 // (warp w owns TMEM lanes 32w..32w+31 = voxel rows), adds the bias, applies
 // ReLU and stores FP32 and/or BF16.
@@ -30,6 +32,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <algorithm>
 
 #include "../../include/fftperm.h"
 #include "common.cuh"
@@ -79,6 +83,14 @@ __device__ __forceinline__ uint64_t smem_desc(const void* p) {
            ((uint64_t)((FP_TC_SBO >> 4) & 0x3FFF) << 32) | (1ull << 46);
 }
 
+// the same for rows 16 bytes apart (eight-row groups 128 bytes apart) and core
+// matrices of neighbouring eight-channel groups `rows` such rows apart
+__device__ __forceinline__ uint64_t smem_desc_rows(const void* p, uint32_t rows) {
+    const uint32_t a = smem_u32(p);
+    return (uint64_t)((a >> 4) & 0x3FFF) | ((uint64_t)(rows & 0x3FFF) << 16) | ((uint64_t)(128 >> 4) << 32) |
+           (1ull << 46);
+}
+
 // instruction descriptor of kind::f16: BF16 A and B, FP32 D, K-major both,
 // N = cout, M = 128
 template <int N>
@@ -99,6 +111,46 @@ __device__ __forceinline__ void tc_fence_after() {
 // ((m / 8) * 2 + q % 2) of 128 bytes, row m % 8 of 16 bytes
 __device__ __forceinline__ uint32_t core_offset(int m, int q, int rows) {
     return (uint32_t)((q >> 1) * rows * 32 + ((m >> 3) * 2 + (q & 1)) * 128 + (m & 7) * 16);
+}
+
+// Sixteen output channels c0.. of a warp's 32 accumulator rows (TMEM lanes from
+// trow): bias, ReLU and the stores of voxel v.
+__device__ __forceinline__ void store_rows(uint32_t trow, int c0, int o0, const float* bias, int relu, bool valid,
+                                           long long v, int cout, float* out32, __nv_bfloat16* out16) {
+    uint32_t rr[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,"
+        "%13,%14,%15}, [%16];"
+        : "=r"(rr[0]), "=r"(rr[1]), "=r"(rr[2]), "=r"(rr[3]), "=r"(rr[4]), "=r"(rr[5]),
+          "=r"(rr[6]), "=r"(rr[7]), "=r"(rr[8]), "=r"(rr[9]), "=r"(rr[10]), "=r"(rr[11]),
+          "=r"(rr[12]), "=r"(rr[13]), "=r"(rr[14]), "=r"(rr[15])
+        : "r"(trow + (uint32_t)c0));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    if (!valid) return;
+    float f[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+        f[j] = __uint_as_float(rr[j]);
+        if (bias) f[j] += bias[o0 + c0 + j];
+        if (relu) f[j] = fmaxf(f[j], 0.f);
+    }
+    if (out32) {
+        float4* o = reinterpret_cast<float4*>(out32 + v * cout + o0 + c0);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o[j] = make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
+    }
+    if (out16) {
+        uint32_t pk[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const uint32_t lo = __bfloat16_as_ushort(__float2bfloat16(f[2 * j]));
+            const uint32_t hi = __bfloat16_as_ushort(__float2bfloat16(f[2 * j + 1]));
+            pk[j] = lo | (hi << 16);
+        }
+        uint4* o = reinterpret_cast<uint4*>(out16 + v * cout + o0 + c0);
+        o[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+        o[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+    }
 }
 
 template <int COUT, int STAGES>
@@ -243,45 +295,157 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_tc(TcConv p) {
         // epilogue: TMEM lanes 32w..32w+31 are the rows of warp w
         const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
 #pragma unroll
-        for (int c0 = 0; c0 < COUT; c0 += 16) {
-            uint32_t rr[16];
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,"
-                "%13,%14,%15}, [%16];"
-                : "=r"(rr[0]), "=r"(rr[1]), "=r"(rr[2]), "=r"(rr[3]), "=r"(rr[4]), "=r"(rr[5]),
-                  "=r"(rr[6]), "=r"(rr[7]), "=r"(rr[8]), "=r"(rr[9]), "=r"(rr[10]), "=r"(rr[11]),
-                  "=r"(rr[12]), "=r"(rr[13]), "=r"(rr[14]), "=r"(rr[15])
-                : "r"(trow + (uint32_t)c0));
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            float f[16];
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                f[j] = __uint_as_float(rr[j]);
-                if (p.bias) f[j] += p.bias[o0 + c0 + j];
-                if (p.relu) f[j] = fmaxf(f[j], 0.f);
-            }
-            if (valid) {
-                if (p.out32) {
-                    float4* o = reinterpret_cast<float4*>(p.out32 + v * p.cout + o0 + c0);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        o[j] = make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
-                }
-                if (p.out16) {
-                    uint32_t pk[8];
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const uint32_t lo = __bfloat16_as_ushort(__float2bfloat16(f[2 * j]));
-                        const uint32_t hi = __bfloat16_as_ushort(__float2bfloat16(f[2 * j + 1]));
-                        pk[j] = lo | (hi << 16);
-                    }
-                    uint4* o = reinterpret_cast<uint4*>(p.out16 + v * p.cout + o0 + c0);
-                    o[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                    o[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-                }
-            }
-        }
+        for (int c0 = 0; c0 < COUT; c0 += 16) store_rows(trow, c0, o0, p.bias, p.relu, valid, v, p.cout, p.out32, p.out16);
     }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(NCOLS)
+                     : "memory");
+}
+
+// The same convolution (dilation 1) with the neighbourhood loaded once per tile.
+// Positions are linear in a sample's volume padded by one voxel along x and y
+// (rows of nx + 2, planes of ny + 2 rows), so the neighbours of 128 consecutive
+// positions in one plane are the same positions shifted by dy (nx + 2) + dx: a
+// CTA copies the 128 + 2 (nx + 3) voxel rows of the three planes z - 1, z, z + 1
+// into shared memory as K-major core matrices with the rows 16 bytes apart
+// (stride byte offset 128, one plane per eight channels), and each tap's A
+// operand is the start address moved by its shift.  All 27 taps' MMAs issue
+// without another barrier, and a voxel's row is read about 4 times per tile
+// position instead of 27 times.  Positions on the padding compute values nobody
+// reads.  The weights stay in shared memory over a CTA's tiles.  Against the per-tap
+// form: four 32^3 cells 16 -> 32 channels 77 -> 35 us, 32 -> 16 116 -> 42, four 64^3
+// cells 16 -> 16 326 -> 126 (the copies into shared memory bound it).
+struct HaloConv {
+    int nx, ny, nz, samples;
+    long long n;
+    int sign;
+    const __nv_bfloat16* in;
+    int cin, cout;
+    const __nv_bfloat16* w;
+    const float* bias;
+    int relu;
+    float* out32;
+    __nv_bfloat16* out16;
+    int pitch, plane;       // nx + 2, (nx + 2) (ny + 2)
+    int rows;               // voxel rows of one plane segment: 128 + 2 (pitch + 1)
+    int tiles;              // tiles per sample
+    long long ntiles;
+};
+
+template <int COUT>
+__global__ void __launch_bounds__(kTcThreads) k_conv_halo(const __grid_constant__ HaloConv p) {
+    constexpr int NCOLS = COUT < 32 ? 32 : COUT;
+    extern __shared__ __align__(1024) unsigned char sm[];
+    uint64_t* bar = reinterpret_cast<uint64_t*>(sm);
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + 64);
+    const int tid = threadIdx.x;
+    const int warp = tid >> 5;
+    const int cin = p.cin;
+    const int kc = cin / 16, per = cin / 8;
+    const int o0 = blockIdx.y * COUT;
+    unsigned char* wsm = sm + 1024;                          // [27][cin/16][COUT * 32 bytes]
+    unsigned char* asm_ = wsm + (size_t)27 * COUT * cin * 2;  // [cin/8][3][rows] 16-byte rows
+    const int seg_rows = 3 * p.rows;
+    const int last = p.nz * p.plane;
+
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                         smem_u32(tslot)),
+                     "r"(NCOLS)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 0) {
+        mbar_init(bar, 1);
+        fence_mbar_init();
+    }
+    // the weights of this CTA's output channels
+    for (int i = tid; i < 27 * COUT * per; i += kTcThreads) {
+        const int tap = i / (COUT * per), e = i - tap * COUT * per;
+        const int co = e / per, q = e - co * per;
+        cp_async16_zfill(wsm + (size_t)tap * COUT * cin * 2 + core_offset(co, q, COUT),
+                         p.w + ((size_t)tap * p.cout + o0 + co) * cin + q * 8, true);
+    }
+    auto load = [&](long long tile) {
+        const int smp = (int)(tile / p.tiles);
+        const int j0 = (int)(tile - (long long)smp * p.tiles) * kTcM;
+        const __nv_bfloat16* in = p.in + (size_t)smp * p.n * cin;
+        for (int r = tid; r < seg_rows; r += kTcThreads) {
+            const int seg = r / p.rows, t = r - seg * p.rows;
+            const int j = j0 - (p.pitch + 1) + t;
+            const bool ok = j >= 0 && j < last;
+            const int jj = ok ? j : 0;
+            int z = jj / p.plane;
+            const int rem = jj - z * p.plane;
+            const int yp = rem / p.pitch, xp = rem - yp * p.pitch;
+            const int y = yp == 0 ? p.ny - 1 : (yp > p.ny ? 0 : yp - 1);
+            const int x = xp == 0 ? p.nx - 1 : (xp > p.nx ? 0 : xp - 1);
+            z += seg - 1;
+            z = z < 0 ? p.nz - 1 : (z >= p.nz ? 0 : z);
+            const __nv_bfloat16* src = in + ((size_t)((long long)z * p.ny + y) * p.nx + x) * cin;
+            for (int q = 0; q < per; ++q)
+                cp_async16_zfill(asm_ + ((size_t)q * seg_rows + r) * 16, src + q * 8, ok);
+        }
+    };
+    long long tile = blockIdx.x;
+    if (tile < p.ntiles) load(tile);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tslot;
+
+    bool ok = true;
+    for (uint32_t it = 0; tile < p.ntiles; tile += gridDim.x, ++it) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        fence_proxy_async_smem();
+        tc_fence_before();  // the epilogue's TMEM reads of the tile before
+        __syncthreads();
+        if (tid == 0) {
+            tc_fence_after();
+            for (int tap = 0; tap < 27; ++tap) {
+                const int dz = p.sign * (tap / 9 - 1), sh = p.sign * ((tap / 3 % 3 - 1) * p.pitch + tap % 3 - 1);
+                const unsigned char* a = asm_ + ((size_t)(dz + 1) * p.rows + p.pitch + 1 + sh) * 16;
+                const unsigned char* bm = wsm + (size_t)tap * COUT * cin * 2;
+                for (int k = 0; k < kc; ++k) {
+                    const uint64_t ad = smem_desc_rows(a + (size_t)2 * k * seg_rows * 16, (uint32_t)seg_rows);
+                    const uint64_t bd = smem_desc(bm + (size_t)k * COUT * 32);
+                    const uint32_t acc = (tap | k) != 0;
+                    asm volatile(
+                        "{\n"
+                        " .reg .pred p;\n"
+                        " setp.ne.b32 p, %4, 0;\n"
+                        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+                        "}\n" ::"r"(tmem),
+                        "l"(ad), "l"(bd), "r"(idesc_bf16<COUT>()), "r"(acc)
+                        : "memory");
+                }
+            }
+            asm volatile(
+                "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
+                : "memory");
+        }
+        // the position of this thread's accumulator row, while the MMAs run
+        const int smp = (int)(tile / p.tiles);
+        const int j = (int)(tile - (long long)smp * p.tiles) * kTcM + tid;
+        const int z = j / p.plane, rem = j - z * p.plane;
+        const int yp = rem / p.pitch, xp = rem - yp * p.pitch;
+        const bool valid = j < last && yp >= 1 && yp <= p.ny && xp >= 1 && xp <= p.nx;
+        const long long v = smp * p.n + ((long long)z * p.ny + yp - 1) * p.nx + xp - 1;
+        ok = mbar_wait_bounded(bar, it & 1u);
+        if (__syncthreads_or(!ok)) {
+            ok = false;
+            if (tid == 0) atomicExch(&g_tc_err, 1);
+            break;
+        }
+        tc_fence_after();
+        if (tile + gridDim.x < p.ntiles) load(tile + gridDim.x);  // the MMAs have read this tile's rows
+        const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
+#pragma unroll
+        for (int c0 = 0; c0 < COUT; c0 += 16) store_rows(trow, c0, o0, p.bias, p.relu, valid, v, p.cout, p.out32, p.out16);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     tc_fence_before();
     __syncthreads();
     if (warp == 0)
@@ -329,6 +493,64 @@ extern "C" int fp_nn_conv_tc(int nx, int ny, int nz, int64_t total, int dilation
     if (blocks > 0x7fffffffLL) return FP_ERR_INVALID;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (cout != 16 && cout != 32 && cout != 64 && cout != 128) return FP_ERR_INVALID;
+    {
+        // The tile form takes dilation 1, up to 64 input channels (their rows and
+        // weights fit shared memory) and samples that 32-bit positions cover.  Its
+        // output channels are split until two CTAs fit an SM, or else one.
+        fp::HaloConv h{};
+        h.nx = nx;
+        h.ny = ny;
+        h.nz = nz;
+        h.samples = (int)(p.total / p.n);
+        h.n = p.n;
+        h.sign = sign;
+        h.in = p.in;
+        h.cin = cin;
+        h.cout = cout;
+        h.w = p.w;
+        h.bias = bias;
+        h.relu = relu;
+        h.out32 = p.out32;
+        h.out16 = p.out16;
+        const long long pitch = nx + 2, plane = pitch * (ny + 2), vol = plane * nz;
+        const long long rows = fp::kTcM + 2 * (pitch + 1);
+        auto need = [&](int t) { return 1024 + (size_t)27 * t * cin * 2 + (size_t)3 * rows * cin * 2; };
+        int t = cout;
+        while (t > 16 && need(t) > 113 * 1024) t /= 2;
+        if (need(t) > 113 * 1024)
+            for (t = cout; t > 16 && need(t) > 226 * 1024;) t /= 2;
+        if (dilation == 1 && cin <= 64 && vol < (1LL << 30) && 3 * rows <= 0x3FFF && need(t) <= 226 * 1024 &&
+            p.total / p.n < (1LL << 30)) {
+            h.pitch = (int)pitch;
+            h.plane = (int)plane;
+            h.rows = (int)rows;
+            h.tiles = (int)((vol + fp::kTcM - 1) / fp::kTcM);
+            h.ntiles = (long long)h.tiles * h.samples;
+            const size_t share = (size_t)233472 * (t < 32 ? 32 : t) / 512;
+            const size_t hs = need(t) > share ? need(t) : share;
+            int dev = 0, sms = 152;
+            cudaGetDevice(&dev);
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            const long long fit = std::min<long long>(16, 232448 / (long long)(hs + 1024));
+            const unsigned splits = (unsigned)(cout / t);
+            const unsigned gx = (unsigned)std::min<long long>(h.ntiles, std::max<long long>(1, fit * sms / splits));
+#define FP_HALO_LAUNCH(C)                                                                \
+    {                                                                                    \
+        static std::atomic<unsigned long long> done_{0};                                 \
+        fp::ensure_smem_limit(fp::k_conv_halo<C>, done_);                                \
+        FP_LAUNCHED();                                                                   \
+        fp::k_conv_halo<C><<<dim3(gx, splits), fp::kTcThreads, hs, s>>>(h);              \
+    }
+            switch (t) {
+                case 16: FP_HALO_LAUNCH(16) break;
+                case 32: FP_HALO_LAUNCH(32) break;
+                case 64: FP_HALO_LAUNCH(64) break;
+                default: FP_HALO_LAUNCH(128) break;
+            }
+#undef FP_HALO_LAUNCH
+            return cudaGetLastError() == cudaSuccess ? FP_OK : FP_ERR_CUDA;
+        }
+    }
     // Output channels per CTA: all of them (the gathered rows serve them all)
     // while the voxels alone give two CTAs per SM; fewer voxels, as on the
     // coarse levels, split the channels down to 32.

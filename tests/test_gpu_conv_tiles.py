@@ -1,4 +1,6 @@
-"""fp_nn_conv_tc on grids large enough for all output channels in one CTA and
+"""fp_nn_conv_tc's tile form (dilation 1, up to 64 input channels: planes of less
+and more than a tile, edges of one voxel, several samples, both signs) and its
+per-tap form, the latter on grids large enough for all output channels in one CTA and
 small enough to split them (the launch rule of learned_tc.cu), with three and
 four buffers, against a float64 convolution."""
 import ctypes as C
@@ -9,7 +11,9 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("cin,cout", [(16, 16), (16, 32), (32, 64), (64, 32), (64, 128), (128, 64), (128, 128), (112, 64)])
-@pytest.mark.parametrize("shape,samples,dil,sign", [((32, 32, 40), 1, 1, 1), ((20, 16, 33), 4, 2, -1), ((9, 5, 3), 1, 1, 1)])
+@pytest.mark.parametrize("shape,samples,dil,sign", [((32, 32, 40), 1, 1, 1), ((20, 16, 33), 4, 2, -1), ((9, 5, 3), 1, 1, 1),
+                                                     ((20, 16, 33), 2, 1, -1), ((1, 7, 2), 3, 1, -1), ((3, 1, 1), 2, 1, 1),
+                                                     ((6, 4, 130), 1, 1, 1)])
 def test_conv_tiles(gpu_lib, cin, cout, shape, samples, dil, sign):
     import torch
 
