@@ -196,9 +196,9 @@ int device_operator_apply(Problem& P, const double* d_x, double* d_y) {
     a.dst = d_y;
     a.src_kind = fp::kSrcCompact;
     a.dst_kind = fp::kDstCompact;
+    a.sum_out = P.d_red + 4;
     int nparts = 0;
     FP_CUDA(fp::launch_apply(P, a, &nparts), "apply");
-    FP_CUDA(fp::launch_reduce4(P, nparts, P.d_red + 4), "reduce");
     FP_CUDA(fp::launch_sub_mean(P, d_y, P.d_red + 4, 1.0), "sub_mean");
     return FP_OK;
 }
@@ -219,9 +219,9 @@ int device_build_rhs(Problem& P, const double g[3], double* d_b) {
     a.dst = d_b;
     a.src_kind = fp::kSrcF0;
     a.dst_kind = fp::kDstCompact;
+    a.sum_out = P.d_red + 4;
     int nparts = 0;
     FP_CUDA(fp::launch_apply(P, a, &nparts), "apply");
-    FP_CUDA(fp::launch_reduce4(P, nparts, P.d_red + 4), "reduce");
     FP_CUDA(fp::launch_sub_mean(P, d_b, P.d_red + 4, -1.0), "sub_mean");
     return FP_OK;
 }
@@ -237,9 +237,9 @@ int residual_norm(Problem& P, const double* d_b, const double* d_y, int precisio
     a.src_kind = fp::kSrcCompact;
     a.dst_kind = fp::kDstCompact;
     a.precision = precision;
+    a.sum_out = P.d_red + 4;
     int nparts = 0;
     FP_CUDA(fp::launch_apply(P, a, &nparts), "apply");
-    FP_CUDA(fp::launch_reduce4(P, nparts, P.d_red + 4), "reduce");
     FP_CUDA(fp::launch_sub_mean(P, P.d_cout, P.d_red + 4, 1.0), "sub_mean");
     FP_CUDA(fp::launch_resnorm(P, d_b, P.d_cout, P.d_red + 12), "resnorm");
     double h[4];
@@ -468,9 +468,9 @@ int device_recover(Problem& P, const double g[3], const double* d_x, double avg[
     a.dst = P.d_dense_out;
     a.src_kind = fp::kSrcF0Compact;
     a.dst_kind = fp::kDstDense;
+    a.sum_out = P.d_red + 4;  // sums over all voxels
     int nparts = 0;
     FP_CUDA(fp::launch_apply(P, a, &nparts), "apply");
-    FP_CUDA(fp::launch_reduce4(P, nparts, P.d_red + 4), "reduce");  // sums over all voxels
     FP_CUDA(fp::launch_gather_sum(P, P.d_dense_out, P.d_red + 8), "gather_sum");
     double h[12];
     FP_CUDA(cudaMemcpyAsync(h, P.d_red, sizeof(double) * 12, cudaMemcpyDeviceToHost, P.stream),

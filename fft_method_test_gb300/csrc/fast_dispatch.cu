@@ -135,7 +135,8 @@ cudaError_t fast_plan(Problem& P, const ApplyArgs& aa, FastPlan<T>& pl) {
     a.skip = aa.skip;
     a.err = P.d_err;
     a.alpha_sc = aa.alpha_sc;
-    a.alpha_ticket = aa.alpha_ticket;
+    a.alpha_ticket = aa.sum_out ? reinterpret_cast<unsigned int*>(P.d_red + kTicketSlot) + 2 : aa.alpha_ticket;
+    a.sum_out = aa.sum_out;
 
     // x passes: tiles of `rows` grid rows, persistent over the tiles
     // grid rows per tile: the tuned cap when set (even), else about 192 threads

@@ -401,6 +401,7 @@ struct FastArgs {
     // Lanczos alpha (null: the caller reduces them)
     MinresScalars* alpha_sc;
     unsigned int* alpha_ticket;
+    double* sum_out;  // or to their four sums (null: the caller reduces them)
     // A group of problems of one grid in one launch per pass: when set, the
     // kernels (GROUP = true) take their member's arguments from group[p], p =
     // blockIdx.y (x and z passes) or blockIdx.z / 3 (y pass), and the z pass
@@ -748,8 +749,14 @@ __global__ void __launch_bounds__(384) k_fx_inv(const __grid_constant__ FastArgs
 #pragma unroll
         for (int i = 0; i < 4; ++i) a.partials[4LL * blockIdx.x + i] = out[i];
     }
-    if (a.alpha_sc && last_block(a.alpha_ticket, gridDim.x))
-        alpha_body(a.alpha_sc, a.partials, (int)gridDim.x, a.inv_nb, red);
+    if (a.alpha_sc) {
+        if (last_block(a.alpha_ticket, gridDim.x))
+            alpha_body(a.alpha_sc, a.partials, (int)gridDim.x, a.inv_nb, red);
+    } else if (a.sum_out && last_block(a.alpha_ticket, gridDim.x)) {
+        sum_rows<4, 4>(a.partials, (int)gridDim.x, red, out);
+        if (threadIdx.x == 0)
+            for (int i = 0; i < 4; ++i) a.sum_out[i] = out[i];
+    }
 }
 
 // ---- P2 / P4: y pass -------------------------------------------------------------

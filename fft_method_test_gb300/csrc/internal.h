@@ -164,7 +164,8 @@ struct Problem {
 
 constexpr int kMaxPartials = 8192;
 // d_red slot (in doubles) holding the block-count tickets of the fused MINRES
-// kernels (z update, v/w update, alpha: three unsigned ints, zero between launches)
+// kernels (z update, v/w update, inverse x pass, vector sums: four unsigned ints,
+// zero between launches)
 constexpr int kTicketSlot = 56;
 
 // ---- setup kernels (kernels_setup.cu) ----
@@ -245,6 +246,9 @@ struct ApplyArgs {
     // mean and alpha from the partial rows (both set, or both null)
     MinresScalars* alpha_sc = nullptr;
     unsigned int* alpha_ticket = nullptr;
+    // device: receives the sums of the partial rows (4); a reduction kernel
+    // after the passes where the inverse x pass's last block does not form them
+    double* sum_out = nullptr;
 };
 
 // Runs the five passes (forward x, y, z + Green + inverse z, inverse y,

@@ -464,8 +464,8 @@ cudaError_t launch_apply(Problem& P, const ApplyArgs& a, int* nparts) {
     if (prec != kFP64 && !P.d_green32) return cudaErrorInvalidValue;
     if (fast_apply_supported(P, prec, a.src_kind, a.dst_kind, a.stage))
         return fast_apply(P, prec, a, nparts);
-    if (prec == kFP64) return apply_impl<double>(P, a, nparts);
-    return apply_impl<float>(P, a, nparts);
+    const cudaError_t e = prec == kFP64 ? apply_impl<double>(P, a, nparts) : apply_impl<float>(P, a, nparts);
+    return e == cudaSuccess && a.sum_out ? launch_reduce4(P, *nparts, a.sum_out) : e;
 }
 
 }  // namespace fp

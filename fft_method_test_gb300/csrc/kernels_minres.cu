@@ -52,7 +52,8 @@ int iter_threads(const Problem& P) {
 // the component of every load static; the odd tail voxel goes to the first
 // thread of block 0.
 template <bool SQUARES>
-__global__ void k_sum3(const double* v, long long nb, double* partials) {
+__global__ void k_sum3(const double* v, long long nb, double* partials, double* out4,
+                       unsigned int* ticket) {
     pdl_wait();
     __shared__ double red[4 * 32];
     double acc[4] = {0, 0, 0, 0};
@@ -79,6 +80,12 @@ __global__ void k_sum3(const double* v, long long nb, double* partials) {
     block_sum<4>(acc, red, out);
     if (threadIdx.x == 0)
         for (int i = 0; i < 4; ++i) partials[4LL * blockIdx.x + i] = out[i];
+    // with out4 the last block reduces the partial rows as well
+    if (out4 && last_block(ticket, gridDim.x)) {
+        sum_rows<4, 4>(partials, (int)gridDim.x, red, out);
+        if (threadIdx.x == 0)
+            for (int i = 0; i < 4; ++i) out4[i] = out[i];
+    }
 }
 
 __global__ void k_reduce4(const double* partials, int nparts, double* out) {
@@ -376,10 +383,11 @@ __global__ void k_axpby(double* out, double a, const double* x, double b,
 
 }  // namespace
 
+static unsigned int* sum_ticket(Problem& P) { return reinterpret_cast<unsigned int*>(P.d_red + kTicketSlot) + 3; }
+
 cudaError_t launch_sum3(Problem& P, const double* v, long long nb, double* out4) {
     const int blocks = vec_blocks(P, (nb + 1) / 2);
-    launch_pdl(k_sum3<false>, blocks, kVecThreads, 0, P.stream, v, nb, P.d_partials);
-    launch_pdl(k_reduce4, 1, 256, 0, P.stream, P.d_partials, blocks, out4);
+    launch_pdl(k_sum3<false>, blocks, kVecThreads, 0, P.stream, v, nb, P.d_partials, out4, sum_ticket(P));
     return cudaGetLastError();
 }
 
@@ -404,7 +412,7 @@ cudaError_t minres_start(Problem& P, const double* b, const double* x0, double t
     if (e != cudaSuccess) return e;
     const int blocks = vec_blocks(P, m);
     // |b|
-    launch_pdl(k_sum3<true>, blocks, kVecThreads, 0, P.stream, b, P.nb, P.d_partials);
+    launch_pdl(k_sum3<true>, blocks, kVecThreads, 0, P.stream, b, P.nb, P.d_partials, nullptr, nullptr);
     launch_pdl(k_start_norms, 1, 256, 0, P.stream, P.d_sc, P.d_partials, blocks, 0);
     // x = x0 or 0
     if (x0) {
@@ -433,7 +441,7 @@ cudaError_t minres_start(Problem& P, const double* b, const double* x0, double t
         launch_pdl(k_residual0, blocks, kVecThreads, 0, P.stream, P.d_sc, b, P.d_z, nullptr, m, 0);
     }
     // beta1 = |r0|
-    launch_pdl(k_sum3<true>, blocks, kVecThreads, 0, P.stream, P.d_z, P.nb, P.d_partials);
+    launch_pdl(k_sum3<true>, blocks, kVecThreads, 0, P.stream, P.d_z, P.nb, P.d_partials, nullptr, nullptr);
     launch_pdl(k_start_norms, 1, 256, 0, P.stream, P.d_sc, P.d_partials, blocks, 1);
     e = cudaMemcpyAsync(P.h_sc, P.d_sc, sizeof(MinresScalars), cudaMemcpyDeviceToHost, P.stream);
     if (e != cudaSuccess) return e;
@@ -476,8 +484,8 @@ cudaError_t minres_start(Problem& P, const double* b, const double* x0, double t
     cudaMemsetAsync(P.d_w[0], 0, sizeof(double) * m, P.stream);
     cudaMemsetAsync(P.d_w[1], 0, sizeof(double) * m, P.stream);
     // component sums of v (input mean of the first apply)
-    launch_pdl(k_sum3<false>, blocks, kVecThreads, 0, P.stream, P.d_v[0], P.nb, P.d_partials);
-    launch_pdl(k_reduce4, 1, 256, 0, P.stream, P.d_partials, blocks, P.d_red + 8);
+    launch_pdl(k_sum3<false>, blocks, kVecThreads, 0, P.stream, P.d_v[0], P.nb, P.d_partials, P.d_red + 8,
+               sum_ticket(P));
     // copy the three sums into sc->vsum
     cudaMemcpyAsync(&P.d_sc->vsum[0], P.d_red + 8, sizeof(double) * 3, cudaMemcpyDeviceToDevice,
                     P.stream);
