@@ -142,6 +142,13 @@ cudaError_t fast_plan(Problem& P, const ApplyArgs& aa, FastPlan<T>& pl) {
     // grid rows per tile: the tuned cap when set (even), else about 192 threads
     int rows = P.x_rows > 0 ? std::max(2, P.x_rows & ~1) : fast::x_rows_for(P.nx);
     rows = std::min(rows, 2 * fast::kMaxXLines / 3);
+    // FP64 on small grids: shorter tiles until every other SM has one (32^3 has 32
+    // tiles of 32 rows, and the FP64 pipe of the SMs they reach bounds the pass).
+    // Per FP64 iteration at 32^3 62.8 -> 59.3 us, at 48^3 94 -> 86; one tile per SM
+    // gives 64.7 and 89.6, and FP32 passes, bound by latency, only lose (32^3 mixed
+    // apply 14.7 -> 16.6 us).
+    if (sizeof(T) == 8 && P.x_rows <= 0)
+        while (rows > 4 && (P.nrows + rows - 1) / rows < P.sm_count / 2) rows = std::max(4, (rows / 2) & ~1);
     if (rows > P.nrows) rows = (int)((P.nrows + 1) & ~1LL);
     a.rows = rows;
     a.ntiles = (P.nrows + rows - 1) / rows;
