@@ -141,7 +141,10 @@ int fp_recover(fp_handle h, const double grad[3], const double* x, double* v_soa
 int fp_solve_load_case(fp_handle h, const double grad[3], const double* x0, double tol,
                        int64_t maxit, double avg[3], double* x_out, fp_solver_stats* stats);
 /* Three unit load cases and the K assembly of PermeabilityRunner::run
- * (src/app/PermeabilityRunner.cpp:700-777): K[row*3+col] = mu <v_row>^(col). */
+ * (src/app/PermeabilityRunner.cpp:700-777): K[row*3+col] = mu <v_row>^(col).
+ * Up to 160^3 voxels the three cases iterate in lockstep, as in
+ * fp_solve_permeability_block, where the memory for it is there; each case's
+ * stats->seconds is then a third of the call's time. */
 int fp_solve_permeability(fp_handle h, double tol, int64_t maxit, double K[9],
                           fp_solver_stats stats[3]);
 
