@@ -1,0 +1,28 @@
+// launch_rules.h -- host rules of launches that no single GPU can show at work
+// (a second device in the process): plain C++, so that a host program can run
+// them against stand-ins for the CUDA calls.
+#pragma once
+
+#include <atomic>
+
+namespace fp {
+
+// Blocks per cluster of a kernel on device `dev`: 16 where the device lets the
+// kernel exceed the portable 8 (`allow` sets the function attribute, which
+// belongs to one device, and returns whether it took) and `fits` says that it can
+// place such a cluster, else the largest of 8, 4, 2, 1 that it can place.  The
+// answer is kept per device (0: not asked yet); two threads that ask at once get
+// the same one.
+constexpr int kClusterDevices = 64;
+template <class Allow, class Fits>
+int cluster_blocks(std::atomic<int> (&known)[kClusterDevices], int dev, Allow allow, Fits fits) {
+    const bool keep = dev >= 0 && dev < kClusterDevices;
+    if (keep)
+        if (const int n = known[dev].load(std::memory_order_acquire)) return n;
+    int n = allow() ? 16 : 8;
+    while (n > 1 && !fits(n)) n /= 2;
+    if (keep) known[dev].store(n, std::memory_order_release);
+    return n;
+}
+
+}  // namespace fp

@@ -26,6 +26,7 @@
 #include <cooperative_groups.h>
 
 #include "common.cuh"
+#include "launch_rules.h"
 #include "wgrad.cuh"
 
 namespace fp {
@@ -481,20 +482,38 @@ extern "C" int fp_nn_bias_grad(const void* dy_bf16, int64_t total, int cout, flo
         // as many blocks as have four reads per thread to do, at most a cluster of 16
         // (four 64^3 cells with 16 channels: 81 us with 8 blocks and four reads in
         // flight per thread, 45 with 16 and eight)
-        static const bool wide = cudaFuncSetAttribute(fp::k_bias_grad_cluster,
-                                                      cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
-        int blocks = wide ? 16 : 8;
-        while (blocks > 1 && (long long)total * pieces < 4LL * fp::kBgThreads * blocks) blocks /= 2;
         cudaLaunchAttribute attr{};
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = (unsigned)blocks;
-        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
         cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3((unsigned)blocks);
-        cfg.blockDim = dim3(fp::kBgThreads);
-        cfg.stream = static_cast<cudaStream_t>(stream);
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
+        auto cluster = [&](int n) {
+            attr.id = cudaLaunchAttributeClusterDimension;
+            attr.val.clusterDim.x = (unsigned)n;
+            attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+            cfg.gridDim = dim3((unsigned)n);
+            cfg.blockDim = dim3(fp::kBgThreads);
+            cfg.stream = static_cast<cudaStream_t>(stream);
+            cfg.attrs = &attr;
+            cfg.numAttrs = 1;
+        };
+        auto took = [](cudaError_t e) {
+            if (e != cudaSuccess) cudaGetLastError();  // a refusal here is not the call's error
+            return e == cudaSuccess;
+        };
+        static std::atomic<int> known[fp::kClusterDevices];
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess) return FP_ERR_CUDA;
+        int blocks = fp::cluster_blocks(
+            known, dev,
+            [&] {
+                return took(cudaFuncSetAttribute(fp::k_bias_grad_cluster,
+                                                 cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            },
+            [&](int n) {
+                cluster(n);
+                int active = 0;
+                return took(cudaOccupancyMaxActiveClusters(&active, fp::k_bias_grad_cluster, &cfg)) && active > 0;
+            });
+        while (blocks > 1 && (long long)total * pieces < 4LL * fp::kBgThreads * blocks) blocks /= 2;
+        cluster(blocks);
         FP_LAUNCHED();
         return cudaLaunchKernelEx(&cfg, fp::k_bias_grad_cluster, static_cast<const uint4*>(dy_bf16),
                                   (long long)total, pieces, db) == cudaSuccess
