@@ -139,9 +139,10 @@ cudaError_t fast_plan(Problem& P, const ApplyArgs& aa, FastPlan<T>& pl) {
     a.sum_out = aa.sum_out;
 
     // x passes: tiles of `rows` grid rows, persistent over the tiles
-    // grid rows per tile: the tuned cap when set (even), else about 192 threads
+    // grid rows per tile: the tuned cap when set (even; a cap beyond what a CTA
+    // holds asks for no more than that), else about 192 threads
     int rows = P.x_rows > 0 ? std::max(2, P.x_rows & ~1) : fast::x_rows_for(P.nx);
-    rows = std::min(rows, 2 * fast::kMaxXLines / 3);
+    rows = std::min(rows, fast::x_rows_max(P.nx));
     // FP64 on small grids: shorter tiles until every other SM has one (32^3 has 32
     // tiles of 32 rows, and the FP64 pipe of the SMs they reach bounds the pass).
     // Per FP64 iteration at 32^3 62.8 -> 59.3 us, at 48^3 94 -> 86; one tile per SM

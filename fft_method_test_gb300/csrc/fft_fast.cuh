@@ -34,6 +34,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "common.cuh"
@@ -542,8 +543,10 @@ __device__ __forceinline__ void join_lines(T2 (&z)[R1 / TPL][R2], int t, Load& l
 
 // ---- P1: scatter + R2C x -------------------------------------------------------
 
-// complex lines per tile of the x passes at most (3 * rows / 2, rows <= 32)
+// complex lines per tile of the x passes at most (3 * rows / 2, rows <= 32), and
+// threads of a CTA
 constexpr int kMaxXLines = 48;
+constexpr int kMaxXThreads = 384;
 
 // One line's threads share a warp, so the stages of a line exchange through
 // shared memory with warp barriers, and the half spectra leave the registers
@@ -553,7 +556,7 @@ constexpr int kMaxXLines = 48;
 // instructions, 80.3 -> 69.7 us at 256^3 FP32 under ncu; L1 and latency bound
 // it (DRAM at 33 %, 22 warps per SM).
 template <typename T, int N, bool GROUP>
-__global__ void __launch_bounds__(384) k_fx_fwd(const __grid_constant__ FastArgs a0) {
+__global__ void __launch_bounds__(kMaxXThreads) k_fx_fwd(const __grid_constant__ FastArgs a0) {
     pdl_wait();
     __shared__ ArgSlot<GROUP> slot;
     const FastArgs& a = member_args<GROUP>(a0, blockIdx.y, slot);
@@ -656,7 +659,7 @@ __global__ void __launch_bounds__(384) k_fx_fwd(const __grid_constant__ FastArgs
 // form (raw rows staged by cp.async, Hermitian halves read from shared memory):
 // 60 -> 33 M warp instructions, 82.8 -> 70.4 us at 256^3 FP32 under ncu.
 template <typename T, int N, bool GROUP>
-__global__ void __launch_bounds__(384) k_fx_inv(const __grid_constant__ FastArgs a0) {
+__global__ void __launch_bounds__(kMaxXThreads) k_fx_inv(const __grid_constant__ FastArgs a0) {
     pdl_wait();
     __shared__ ArgSlot<GROUP> slot;
     const FastArgs& a = member_args<GROUP>(a0, blockIdx.y, slot);
@@ -1194,6 +1197,13 @@ inline int x_rows_for(int n) {
     }
     const int tpl = x_tpl(n);  // about 192 threads, 96 where a line is long for its threads
     return tpl >= 16 ? 8 : (tpl == 8 || n > 60 ? 16 : 32);
+}
+// grid rows per tile at most (even): the lines of kMaxXLines, and no more than
+// kMaxXThreads threads serve (a line of an edge with 16 threads per line, 240 and
+// 256, takes as many threads as four of 64: 16 rows there, 32 elsewhere)
+inline int x_rows_max(int n) {
+    const int lines = std::min(kMaxXLines, kMaxXThreads / x_tpl(n));
+    return (2 * lines / 3) & ~1;
 }
 template <typename T>
 int x_ld_rt(int n) {
