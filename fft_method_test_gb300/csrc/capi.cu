@@ -1053,7 +1053,7 @@ int group_solve_cases(int count, fp_handle* handles, const int* cols, double tol
     };
     const int chunk = P0.precision == fp::kMixed && P0.reliable_interval > 0 ? P0.reliable_interval : 16;
     {
-        cudaError_t e = fp::group_tables_create(&tab, count, chunk);
+        cudaError_t e = fp::group_tables_create(&tab, count, chunk, P0.stream);
         if (e != cudaSuccess) return restore(cuda_fail(P0, e, "group tables"));
     }
     const double t0 = now_s();

@@ -24,30 +24,39 @@
 
 namespace fp {
 
+// The device tables are stream-ordered allocations and the host ones plain
+// memory: cudaMalloc, cudaMallocHost and their frees may wait for the whole
+// device, and a solve would then stand still behind other streams' kernels (a
+// 32^3 solve of 27 ms beside a kernel of one second took that second).  A chunk
+// copies 60 kB for three members, on a stream that has just been synchronised.
 struct GroupTables {
     int members = 0, iters = 0;
+    cudaStream_t stream = nullptr;
     fast::FastArgs* d_fast = nullptr;  // [iters][members]
     IterArgs* d_iter = nullptr;        // [iters][members]
     CUtensorMap* d_maps = nullptr;     // [members][2]
-    fast::FastArgs* h_fast = nullptr;  // pinned staging of the same
-    IterArgs* h_iter = nullptr;
-    CUtensorMap* h_maps = nullptr;
+    // staging of the same; a copy may still read it until the stream is synchronised
+    std::vector<fast::FastArgs> h_fast;
+    std::vector<IterArgs> h_iter;
+    std::vector<CUtensorMap> h_maps;
 };
 
-cudaError_t group_tables_create(GroupTables** out, int members, int iters) {
+cudaError_t group_tables_create(GroupTables** out, int members, int iters, cudaStream_t stream) {
     *out = nullptr;
     if (members < 1 || iters < 1) return cudaErrorInvalidValue;
     GroupTables* t = new GroupTables;
     t->members = members;
     t->iters = iters;
+    t->stream = stream;
     const size_t nf = (size_t)members * iters;
-    DeviceMemGuard mem_guard;
-    cudaError_t e = cudaMalloc(&t->d_fast, nf * sizeof(fast::FastArgs));
-    if (e == cudaSuccess) e = cudaMalloc(&t->d_iter, nf * sizeof(IterArgs));
-    if (e == cudaSuccess) e = cudaMalloc(&t->d_maps, 2 * (size_t)members * sizeof(CUtensorMap));
-    if (e == cudaSuccess) e = cudaMallocHost(&t->h_fast, nf * sizeof(fast::FastArgs));
-    if (e == cudaSuccess) e = cudaMallocHost(&t->h_iter, nf * sizeof(IterArgs));
-    if (e == cudaSuccess) e = cudaMallocHost(&t->h_maps, 2 * (size_t)members * sizeof(CUtensorMap));
+    t->h_fast.resize(nf);
+    t->h_iter.resize(nf);
+    t->h_maps.resize(2 * (size_t)members);
+    cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&t->d_fast), nf * sizeof(fast::FastArgs), stream);
+    if (e == cudaSuccess)
+        e = cudaMallocAsync(reinterpret_cast<void**>(&t->d_iter), nf * sizeof(IterArgs), stream);
+    if (e == cudaSuccess)
+        e = cudaMallocAsync(reinterpret_cast<void**>(&t->d_maps), t->h_maps.size() * sizeof(CUtensorMap), stream);
     if (e != cudaSuccess) {
         group_tables_destroy(t);
         return e;
@@ -58,13 +67,9 @@ cudaError_t group_tables_create(GroupTables** out, int members, int iters) {
 
 void group_tables_destroy(GroupTables* t) {
     if (!t) return;
-    DeviceMemGuard mem_guard;
-    cudaFree(t->d_fast);
-    cudaFree(t->d_iter);
-    cudaFree(t->d_maps);
-    cudaFreeHost(t->h_fast);
-    cudaFreeHost(t->h_iter);
-    cudaFreeHost(t->h_maps);
+    for (void* p : {(void*)t->d_fast, (void*)t->d_iter, (void*)t->d_maps})
+        if (p) cudaFreeAsync(p, t->stream);
+    cudaStreamSynchronize(t->stream);  // the staging memory goes with t
     delete t;
 }
 
@@ -74,7 +79,7 @@ bool group_supported(Problem& P) {
 }
 
 cudaError_t group_iterations(Problem* const* m, int members, int count, GroupTables* t) {
-    if (members < 1 || count < 1 || !t || members > t->members || count > t->iters)
+    if (members < 1 || count < 1 || !t || members > t->members || count > t->iters || m[0]->stream != t->stream)
         return cudaErrorInvalidValue;
     Problem& P0 = *m[0];
     cudaStream_t s = P0.stream;
@@ -135,13 +140,13 @@ cudaError_t group_iterations(Problem* const* m, int members, int count, GroupTab
         }
     }
     const size_t nf = (size_t)count * members;
-    if ((e = cudaMemcpyAsync(t->d_maps, t->h_maps, 2 * (size_t)members * sizeof(CUtensorMap),
+    if ((e = cudaMemcpyAsync(t->d_maps, t->h_maps.data(), 2 * (size_t)members * sizeof(CUtensorMap),
                              cudaMemcpyHostToDevice, s)) != cudaSuccess)
         return e;
-    if ((e = cudaMemcpyAsync(t->d_fast, t->h_fast, nf * sizeof(fast::FastArgs), cudaMemcpyHostToDevice, s)) !=
-        cudaSuccess)
+    if ((e = cudaMemcpyAsync(t->d_fast, t->h_fast.data(), nf * sizeof(fast::FastArgs), cudaMemcpyHostToDevice,
+                             s)) != cudaSuccess)
         return e;
-    if ((e = cudaMemcpyAsync(t->d_iter, t->h_iter, nf * sizeof(IterArgs), cudaMemcpyHostToDevice, s)) !=
+    if ((e = cudaMemcpyAsync(t->d_iter, t->h_iter.data(), nf * sizeof(IterArgs), cudaMemcpyHostToDevice, s)) !=
         cudaSuccess)
         return e;
     for (int i = 0; i < count; ++i) {

@@ -289,7 +289,7 @@ cudaError_t group_iteration_tail(cudaStream_t s, const IterArgs* d_tab, int memb
 
 // Device tables of a group's lockstep iterations (group.cu).
 struct GroupTables;
-cudaError_t group_tables_create(GroupTables** out, int members, int iters);
+cudaError_t group_tables_create(GroupTables** out, int members, int iters, cudaStream_t stream);
 void group_tables_destroy(GroupTables* t);
 // true when P can be a group member (its applies run the specialised passes)
 bool group_supported(Problem& P);
