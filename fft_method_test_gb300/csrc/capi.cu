@@ -22,6 +22,7 @@
 
 #include "../../include/fftperm.h"
 #include "internal.h"
+#include "launch_rules.h"
 
 std::atomic<long long> fp::g_kernel_launches{0};
 thread_local long long fp::g_thread_launches = 0;
@@ -91,11 +92,13 @@ using fp::Problem;
 
 int fail(Problem& P, int code, const std::string& msg) {
     P.err = msg;
+    P.no_memory = code == FP_ERR_NOMEM;
     return code;
 }
 
 int cuda_fail(Problem& P, cudaError_t e, const char* where) {
     P.err = std::string(where) + ": " + cudaGetErrorString(e);
+    P.no_memory = e == cudaErrorMemoryAllocation;
     return FP_ERR_CUDA;
 }
 
@@ -564,8 +567,12 @@ int fp::create_handle(int nx, int ny, int nz, double voxel_size, double mu, int 
     }
     std::string err;
     if (!fp::make_axis_plan(nx, P.px, err, P.stream) || !fp::make_axis_plan(ny, P.py, err, P.stream) ||
-        !fp::make_axis_plan(nz, P.pz, err, P.stream))
-        return fail(P, FP_ERR_UNSUPPORTED, err);
+        !fp::make_axis_plan(nz, P.pz, err, P.stream)) {
+        const bool memory = cudaGetLastError() == cudaErrorMemoryAllocation;
+        fail(P, FP_ERR_UNSUPPORTED, err);
+        P.no_memory = memory;
+        return FP_ERR_UNSUPPORTED;
+    }
     FP_CUDA(dalloc(P, reinterpret_cast<double2**>(&P.d_spec), 3 * (size_t)fp::spec_capacity(P)),
             "cudaMalloc spec");
     const size_t nparts = (size_t)std::max<long long>(fp::kMaxPartials, P.nrows + 64);
@@ -986,47 +993,6 @@ int fp_solve_load_case(fp_handle h, const double grad[3], const double* x0, doub
     return FP_OK;
 }
 
-int fp_solve_permeability(fp_handle h, double tol, int64_t maxit, double K[9],
-                          fp_solver_stats stats[3]) {
-    if (!h || !K) return FP_ERR_INVALID;
-    Problem& P = h->P;
-    int rc = need_geometry(P, "PermeabilityRunner::run");
-    if (rc) return rc;
-    // Up to 160^3 the three load cases iterate in lockstep (the same K and
-    // iterations): an iteration of a small cell is seven kernels of a few
-    // microseconds, and one launch then serves three of them: FP64 32^3 67 -> 38 ms,
-    // mixed 64^3 48 -> 28, mixed 128^3 185 -> 152 (256^3 1.68 -> 1.60 s).
-    // Larger cells keep the memory of two more sets of vectors for the caller, who
-    // can ask for the block.  When the siblings do not fit, one case at a time.
-    if (P.n <= 160LL * 160 * 160 && fp::group_supported(P)) {
-        const double t0 = now_s();
-        fp_solver_stats st[3];
-        rc = fp_solve_permeability_block(h, tol, maxit, K, st);
-        if (rc != FP_ERR_CUDA && rc != FP_ERR_NOMEM) {
-            for (int c = 0; c < 3 && stats && rc == FP_OK; ++c) {
-                stats[c] = st[c];
-                stats[c].seconds = (now_s() - t0) / 3;  // the cases share the time
-            }
-            return rc;
-        }
-        cudaGetLastError();  // an allocation that failed leaves nothing behind
-        P.err.clear();
-    }
-    for (int col = 0; col < 3; ++col) {
-        double g[3] = {0.0, 0.0, 0.0};
-        g[col] = 1.0;
-        double avg[3];
-        fp_solver_stats st{};
-        rc = fp_solve_load_case(h, g, nullptr, tol, maxit, avg, nullptr, &st);
-        if (rc) return rc;
-        // colK = -mu <v>; set_column stores -colK (PermeabilityRunner.cpp:772-777,
-        // PermeabilityTensor.cpp:16)
-        for (int row = 0; row < 3; ++row) K[row * 3 + col] = -(-P.mu * avg[row]);
-        if (stats) stats[col] = st;
-    }
-    return FP_OK;
-}
-
 }  // extern "C"
 
 namespace {
@@ -1087,70 +1053,40 @@ void set_column(double* K, int col, double mu, const double avg[3]) {
     for (int row = 0; row < 3; ++row) K[row * 3 + col] = -(-mu * avg[row]);
 }
 
-}  // namespace
-
-extern "C" {
-
-int fp_group_solve_permeability(int count, fp_handle* handles, double tol, int64_t maxit, double* K,
-                                fp_solver_stats* stats) {
-    if (count < 1 || !handles || !K) return FP_ERR_INVALID;
-    for (int i = 0; i < count; ++i)
-        if (!handles[i]) return FP_ERR_INVALID;
-    Problem& P0 = handles[0]->P;
-    for (int i = 0; i < count; ++i) {
-        Problem& P = handles[i]->P;
-        int rc = need_geometry(P, "PermeabilityRunner::run");
-        if (rc) return rc;
-        if (P.nx != P0.nx || P.ny != P0.ny || P.nz != P0.nz || P.precision != P0.precision ||
-            P.reliable_interval != P0.reliable_interval)
-            return fail(P, FP_ERR_INVALID, "group: members must share grid, precision and reliable interval");
-        if (P.tile_yz != P0.tile_yz || P.tma_off != P0.tma_off || P.x_bulk != P0.x_bulk ||
-            P.x_rows != P0.x_rows || P.yz_lowreg != P0.yz_lowreg || P.fast_off != P0.fast_off)
-            return fail(P, FP_ERR_INVALID,
-                        "group: members must share the FFT tiling (fp_autotune or fp_set_tiling on each)");
-    }
-    bool grouped = count > 1;
-    for (int i = 0; i < count && grouped; ++i) grouped = fp::group_supported(handles[i]->P);
-    if (!grouped) {  // one at a time on the members' own streams
-        for (int i = 0; i < count; ++i) {
-            int rc = fp_solve_permeability(handles[i], tol, maxit, K + 9 * (size_t)i,
-                                           stats ? stats + 3 * (size_t)i : nullptr);
-            if (rc) return rc;
-        }
-        return FP_OK;
-    }
-    std::vector<int> cols((size_t)count);
-    std::vector<std::array<double, 3>> avg((size_t)count);
-    std::vector<fp_solver_stats> st((size_t)count);
+// The three load cases of h, one after another.
+int solve_one_by_one(fp_handle h, double tol, int64_t maxit, double K[9], fp_solver_stats stats[3]) {
     for (int col = 0; col < 3; ++col) {
-        std::fill(cols.begin(), cols.end(), col);
-        int rc = group_solve_cases(count, handles, cols.data(), tol, maxit,
-                                   reinterpret_cast<double(*)[3]>(avg.data()), st.data());
+        double g[3] = {0.0, 0.0, 0.0};
+        g[col] = 1.0;
+        double avg[3];
+        fp_solver_stats st{};
+        const int rc = fp_solve_load_case(h, g, nullptr, tol, maxit, avg, nullptr, &st);
         if (rc) return rc;
-        for (int i = 0; i < count; ++i) {
-            set_column(K + 9 * (size_t)i, col, handles[i]->P.mu, avg[(size_t)i].data());
-            if (stats) stats[3 * (size_t)i + col] = st[(size_t)i];
-        }
+        set_column(K, col, h->P.mu, avg);
+        if (stats) stats[col] = st;
     }
     return FP_OK;
 }
 
-int fp_solve_permeability_block(fp_handle h, double tol, int64_t maxit, double K[9],
-                                fp_solver_stats stats[3]) {
-    if (!h || !K) return FP_ERR_INVALID;
+// The three load cases of h in lockstep (its grid has specialised passes).
+// *no_memory: the failure is an allocation's.
+int solve_block(fp_handle h, double tol, int64_t maxit, double K[9], fp_solver_stats stats[3], bool* no_memory) {
     Problem& P = h->P;
-    int rc = need_geometry(P, "PermeabilityRunner::run");
-    if (rc) return rc;
-    if (!fp::group_supported(P)) return fp_solve_permeability(h, tol, maxit, K, stats);
+    P.no_memory = false;
     // the Green tables the siblings borrow
-    rc = P.precision == fp::kMixed ? ensure_green_both(P) : ensure_green64(P);
-    if (rc) return rc;
+    int rc = P.precision == fp::kMixed ? ensure_green_both(P) : ensure_green64(P);
+    if (rc) {
+        *no_memory = P.no_memory;
+        return rc;
+    }
     // two siblings: own vectors, spectral buffer and scalars; the same mask,
     // support, tiling and solver settings; the Green tables of h
     fp_handle sib[2] = {nullptr, nullptr};
     auto drop = [&](int code) {
+        *no_memory = code != FP_OK && P.no_memory;
         for (fp_handle s : sib) {
             if (!s) continue;
+            *no_memory = *no_memory || (code != FP_OK && s->P.no_memory);
             s->P.d_green32 = nullptr;  // borrowed
             s->P.d_green64 = nullptr;
             fp_destroy(s);
@@ -1203,6 +1139,96 @@ int fp_solve_permeability_block(fp_handle h, double tol, int64_t maxit, double K
         if (stats) stats[c] = st[c];
     }
     return drop(FP_OK);
+}
+
+}  // namespace
+
+extern "C" {
+
+int fp_group_solve_permeability(int count, fp_handle* handles, double tol, int64_t maxit, double* K,
+                                fp_solver_stats* stats) {
+    if (count < 1 || !handles || !K) return FP_ERR_INVALID;
+    for (int i = 0; i < count; ++i)
+        if (!handles[i]) return FP_ERR_INVALID;
+    Problem& P0 = handles[0]->P;
+    for (int i = 0; i < count; ++i) {
+        Problem& P = handles[i]->P;
+        int rc = need_geometry(P, "PermeabilityRunner::run");
+        if (rc) return rc;
+        if (P.nx != P0.nx || P.ny != P0.ny || P.nz != P0.nz || P.precision != P0.precision ||
+            P.reliable_interval != P0.reliable_interval)
+            return fail(P, FP_ERR_INVALID, "group: members must share grid, precision and reliable interval");
+        if (P.tile_yz != P0.tile_yz || P.tma_off != P0.tma_off || P.x_bulk != P0.x_bulk ||
+            P.x_rows != P0.x_rows || P.yz_lowreg != P0.yz_lowreg || P.fast_off != P0.fast_off)
+            return fail(P, FP_ERR_INVALID,
+                        "group: members must share the FFT tiling (fp_autotune or fp_set_tiling on each)");
+    }
+    bool grouped = count > 1;
+    for (int i = 0; i < count && grouped; ++i) grouped = fp::group_supported(handles[i]->P);
+    if (!grouped) {  // one at a time on the members' own streams
+        for (int i = 0; i < count; ++i) {
+            int rc = fp_solve_permeability(handles[i], tol, maxit, K + 9 * (size_t)i,
+                                           stats ? stats + 3 * (size_t)i : nullptr);
+            if (rc) return rc;
+        }
+        return FP_OK;
+    }
+    std::vector<int> cols((size_t)count);
+    std::vector<std::array<double, 3>> avg((size_t)count);
+    std::vector<fp_solver_stats> st((size_t)count);
+    for (int col = 0; col < 3; ++col) {
+        std::fill(cols.begin(), cols.end(), col);
+        int rc = group_solve_cases(count, handles, cols.data(), tol, maxit,
+                                   reinterpret_cast<double(*)[3]>(avg.data()), st.data());
+        if (rc) return rc;
+        for (int i = 0; i < count; ++i) {
+            set_column(K + 9 * (size_t)i, col, handles[i]->P.mu, avg[(size_t)i].data());
+            if (stats) stats[3 * (size_t)i + col] = st[(size_t)i];
+        }
+    }
+    return FP_OK;
+}
+
+int fp_solve_permeability(fp_handle h, double tol, int64_t maxit, double K[9],
+                          fp_solver_stats stats[3]) {
+    if (!h || !K) return FP_ERR_INVALID;
+    Problem& P = h->P;
+    int rc = need_geometry(P, "PermeabilityRunner::run");
+    if (rc) return rc;
+    // Up to 160^3 the three load cases iterate in lockstep (the same K and
+    // iterations): an iteration of a small cell is seven kernels of a few
+    // microseconds, and one launch then serves three of them: FP64 32^3 67 -> 38 ms,
+    // mixed 64^3 48 -> 28, mixed 128^3 185 -> 152 (256^3 1.68 -> 1.60 s).
+    // Larger cells keep the memory of two more sets of vectors for the caller, who
+    // can ask for the block.  When the siblings do not fit, one case at a time.
+    if (P.n > 160LL * 160 * 160 || !fp::group_supported(P)) return solve_one_by_one(h, tol, maxit, K, stats);
+    return fp::lockstep_or_one_by_one(
+        [&](bool* no_memory) {
+            const double t0 = now_s();
+            fp_solver_stats st[3];
+            const int code = solve_block(h, tol, maxit, K, st, no_memory);
+            for (int c = 0; c < 3 && stats && code == FP_OK; ++c) {
+                stats[c] = st[c];
+                stats[c].seconds = (now_s() - t0) / 3;  // the cases share the time
+            }
+            return code;
+        },
+        [&] {
+            cudaGetLastError();  // the allocation that failed leaves nothing behind
+            P.err.clear();
+            return solve_one_by_one(h, tol, maxit, K, stats);
+        });
+}
+
+int fp_solve_permeability_block(fp_handle h, double tol, int64_t maxit, double K[9],
+                                fp_solver_stats stats[3]) {
+    if (!h || !K) return FP_ERR_INVALID;
+    Problem& P = h->P;
+    int rc = need_geometry(P, "PermeabilityRunner::run");
+    if (rc) return rc;
+    if (!fp::group_supported(P)) return fp_solve_permeability(h, tol, maxit, K, stats);
+    bool no_memory = false;
+    return solve_block(h, tol, maxit, K, stats, &no_memory);
 }
 
 }  // extern "C"

@@ -17,6 +17,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <new>
 #include <vector>
 
 #include "fft_fast.cuh"
@@ -44,14 +45,20 @@ struct GroupTables {
 cudaError_t group_tables_create(GroupTables** out, int members, int iters, cudaStream_t stream) {
     *out = nullptr;
     if (members < 1 || iters < 1) return cudaErrorInvalidValue;
-    GroupTables* t = new GroupTables;
+    const size_t nf = (size_t)members * iters;
+    GroupTables* t = nullptr;
+    try {
+        t = new GroupTables;
+        t->stream = stream;
+        t->h_fast.resize(nf);
+        t->h_iter.resize(nf);
+        t->h_maps.resize(2 * (size_t)members);
+    } catch (const std::bad_alloc&) {
+        delete t;
+        return cudaErrorMemoryAllocation;
+    }
     t->members = members;
     t->iters = iters;
-    t->stream = stream;
-    const size_t nf = (size_t)members * iters;
-    t->h_fast.resize(nf);
-    t->h_iter.resize(nf);
-    t->h_maps.resize(2 * (size_t)members);
     cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&t->d_fast), nf * sizeof(fast::FastArgs), stream);
     if (e == cudaSuccess)
         e = cudaMallocAsync(reinterpret_cast<void**>(&t->d_iter), nf * sizeof(IterArgs), stream);

@@ -160,6 +160,7 @@ struct Problem {
     int* d_err = nullptr;      // device error flag (a bounded wait gave up)
 
     std::string err;
+    bool no_memory = false;    // err stands for an allocation that failed
 };
 
 constexpr int kMaxPartials = 8192;

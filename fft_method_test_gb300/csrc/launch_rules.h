@@ -1,6 +1,6 @@
-// launch_rules.h -- host rules of launches that no single GPU can show at work
-// (a second device in the process): plain C++, so that a host program can run
-// them against stand-ins for the CUDA calls.
+// launch_rules.h -- host rules that a run on one healthy GPU does not show at
+// work (a second device in the process, a device error): plain C++, so that a
+// host program can run them against stand-ins for the CUDA calls.
 #pragma once
 
 #include <atomic>
@@ -23,6 +23,16 @@ int cluster_blocks(std::atomic<int> (&known)[kClusterDevices], int dev, Allow al
     while (n > 1 && !fits(n)) n /= 2;
     if (keep) known[dev].store(n, std::memory_order_release);
     return n;
+}
+
+// The lockstep solve, or where it could not get its memory the load cases one at
+// a time.  Every other failure is the caller's to see: a wait that timed out or a
+// launch that failed in the lockstep is not made good by a second solve.
+template <class Lockstep, class OneByOne>
+int lockstep_or_one_by_one(Lockstep lockstep, OneByOne one_by_one) {
+    bool no_memory = false;
+    const int rc = lockstep(&no_memory);
+    return rc != 0 && no_memory ? one_by_one() : rc;
 }
 
 }  // namespace fp

@@ -1,6 +1,7 @@
 """The launch rules of csrc/launch_rules.h in a host program, with stand-ins for
 the CUDA calls: what a process with a second device, or a device that cannot
-place a large cluster, gets."""
+place a large cluster, gets, and which failures of a lockstep solve are tried again
+one case at a time."""
 import os
 import shutil
 import subprocess
@@ -33,6 +34,14 @@ int main() {
     std::printf("%d", asked);
     static std::atomic<int> none[fp::kClusterDevices];
     std::printf(" %d", fp::cluster_blocks(none, 200, [] { return true; }, [](int) { return false; }));
+    // {code, an allocation failed}: done, a device error, no memory (two codes), not converged
+    const int codes[][2] = {{0, 0}, {3, 0}, {3, 1}, {5, 1}, {2, 0}};
+    for (auto& c : codes) {
+        int again = 0;
+        const int rc = fp::lockstep_or_one_by_one(
+            [&](bool* no_memory) { return *no_memory = c[1], c[0]; }, [&] { return ++again, 0; });
+        std::printf(" %d%d", rc, again);
+    }
 }
 """
 
@@ -63,3 +72,7 @@ def test_bias_gradient_keeps_no_process_wide_attribute():
     body = src[src.index("fp_nn_bias_grad("):]
     body = body[:body.index("\n}")]
     assert "cluster_blocks(" in body and "static const bool" not in body
+
+
+def test_only_a_lack_of_memory_is_tried_again(program):
+    assert program.split()[10:] == ["00", "30", "01", "01", "20"]
