@@ -77,22 +77,27 @@ void apply_tiling(Problem& P, int tile, bool tma_off, bool x_bulk, int x_rows, b
 
 // Mean time of `reps` operator applies (compact source when a geometry is
 // set, dense otherwise) on the handle's stream, after one warm-up apply.
+// Compact applies are timed with what a MINRES iteration adds to them for
+// alpha, on either path: the dot with the source and the reduction of the partial
+// rows, by the last block of the specialised inverse x pass or by a kernel after
+// the generic passes.  Its length depends on the tiling (many small x tiles make
+// many rows), and a candidate timed without it would win by what it leaves out.
 int time_apply(Problem& P, int reps, double* ms) {
     ApplyArgs a;
+    bool alpha_kernel = false;
     if (P.has_geometry && P.nb > 0) {
         cudaMemsetAsync(P.d_x, 0, sizeof(double) * 3 * (size_t)P.nb, P.stream);
+        cudaMemsetAsync(P.d_sc, 0, sizeof(MinresScalars), P.stream);
         a.src = P.d_x;
         a.dst = P.d_cout;
         a.src_kind = kSrcCompact;
         a.dst_kind = kDstCompact;
-        // with the reduction to alpha that MINRES has the inverse x pass do: its
-        // length depends on the tiling (many small x tiles make many partial
-        // rows for one small last block)
+        a.dot_with = P.d_x;
         if (fast_apply_supported(P, P.precision, a.src_kind, a.dst_kind, a.stage)) {
-            cudaMemsetAsync(P.d_sc, 0, sizeof(MinresScalars), P.stream);
-            a.dot_with = P.d_x;
             a.alpha_sc = P.d_sc;
             a.alpha_ticket = reinterpret_cast<unsigned int*>(P.d_red + kTicketSlot) + 2;
+        } else {
+            alpha_kernel = true;
         }
     } else {
         if (!P.d_dense_in && cudaMallocAsync(reinterpret_cast<void**>(&P.d_dense_in),
@@ -107,14 +112,18 @@ int time_apply(Problem& P, int reps, double* ms) {
         a.src_kind = kSrcDense;
         a.dst_kind = kDstDense;
     }
-    int np = 0;
-    if (launch_apply(P, a, &np) != cudaSuccess) return FP_ERR_CUDA;
+    auto apply = [&]() -> cudaError_t {
+        int np = 0;
+        const cudaError_t e = launch_apply(P, a, &np);
+        return e == cudaSuccess && alpha_kernel ? launch_alpha(P, np) : e;
+    };
+    if (apply() != cudaSuccess) return FP_ERR_CUDA;
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     cudaEventRecord(e0, P.stream);
     cudaError_t err = cudaSuccess;
-    for (int i = 0; i < reps && err == cudaSuccess; ++i) err = launch_apply(P, a, &np);
+    for (int i = 0; i < reps && err == cudaSuccess; ++i) err = apply();
     cudaEventRecord(e1, P.stream);
     cudaEventSynchronize(e1);
     float t = 0.f;

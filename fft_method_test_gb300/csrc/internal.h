@@ -303,6 +303,9 @@ cudaError_t group_iterations(Problem* const* m, int members, int count, GroupTab
 cudaError_t launch_sum3(Problem& P, const double* v, long long nb, double* out3);
 // Reduce [nparts][4] partials into out4 (deterministic, one block).
 cudaError_t launch_reduce4(Problem& P, int nparts, double* out4);
+// z mean and alpha from the apply's partial rows, for applies whose last block
+// does not form them
+cudaError_t launch_alpha(Problem& P, int nparts);
 // r0_precision: operator precision of r0 = b - A x0 (-1: the problem's own);
 // ax0: A x0 with its mean removed where the caller has it, or null
 cudaError_t minres_start(Problem& P, const double* b, const double* x0, double tol,

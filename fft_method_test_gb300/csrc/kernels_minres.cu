@@ -600,6 +600,11 @@ cudaError_t group_iteration_tail(cudaStream_t s, const IterArgs* d_tab, int memb
     return cudaGetLastError();
 }
 
+cudaError_t launch_alpha(Problem& P, int nparts) {
+    launch_pdl(k_alpha, 1, 512, 0, P.stream, P.d_sc, P.d_partials, nparts, 1.0 / (double)P.nb);
+    return cudaGetLastError();
+}
+
 cudaError_t minres_iteration(Problem& P) {
     IterArgs t;
     ApplyArgs a;
@@ -607,7 +612,7 @@ cudaError_t minres_iteration(Problem& P) {
     int nparts = 0;
     cudaError_t e = launch_apply(P, a, &nparts);
     if (e != cudaSuccess) return e;
-    if (!a.alpha_sc) launch_pdl(k_alpha, 1, 512, 0, P.stream, t.sc, t.partials, nparts, t.inv_nb);
+    if (!a.alpha_sc && (e = launch_alpha(P, nparts)) != cudaSuccess) return e;
     // the last block of k_zupd runs the Givens step, the last block of
     // k_vwupd the end of the iteration (block-count tickets in d_red)
     launch_pdl(k_zupd, t.nblk, t.threads, 0, P.stream, t.sc, t.z, t.v, t.v_old, t.nb, t.partials,
