@@ -11,8 +11,7 @@
 // count, so every member computes exactly what it computes alone.  When all
 // members share one Green table (same grid, voxel size, viscosity and alias
 // radius), the z pass is k_fz_shared, which loads each Green tile once for
-// all members (and transforms a done member's stale spectrum, which nothing
-// reads, rather than skip it).
+// all members (and leaves done members out as well).
 #include <cuda_runtime.h>
 
 #include <algorithm>
