@@ -5,6 +5,7 @@
 #include <algorithm>
 
 #include "fft_fast.cuh"
+#include "launch_rules.h"
 
 namespace fp {
 namespace fast {
@@ -81,9 +82,9 @@ int x_blocks_per_sm(int n, bool inverse, int threads, size_t smem) {
 }  // namespace fast
 
 bool fast_apply_supported(const Problem& P, int precision, int src_kind, int dst_kind, int stage) {
-    (void)precision;
     if (P.fast_off || P.tma_off || !P.d_err) return false;
     if (src_kind != kSrcCompact || dst_kind != kDstCompact || stage != kStageFull) return false;
+    if (precision == kFP64 && fp64_generic_passes(P.nx, P.ny, P.nz)) return false;
     return fast::edge_supported(P.nx) && fast::edge_supported(P.ny) && fast::edge_supported(P.nz);
 }
 

@@ -979,7 +979,7 @@ __global__ void __launch_bounds__(3 * TX * Split<N>::TPL, STAGES == 1 ? 3 : 1)
 // and the items after it are those of the `na` active members; that first item is
 // waited for and not transformed when member 0 is done.  (With done
 // members transformed to the end of their chunk, 20 iterations of three FP64 load
-// cases at 200 x 200 x 100 took 226 ms, without 183; 100 at 128^3 289 and 278.)
+// cases at 100 x 200 x 200 took 226 ms, without 183; 100 at 128^3 289 and 278.)
 // Waits are bounded: on a timeout member 0's error flag is raised.
 constexpr int kActiveMembers = 64;  // larger groups transform every member
 template <typename T, int N, int TX>

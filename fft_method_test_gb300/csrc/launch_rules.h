@@ -35,4 +35,18 @@ int lockstep_or_one_by_one(Lockstep lockstep, OneByOne one_by_one) {
     return rc != 0 && no_memory ? one_by_one() : rc;
 }
 
+// FP64 operator applies that stay with the generic passes although their grid has
+// specialised ones: z = 162 with y one of 162, 200, 216, and grids of these edges
+// alone.  The FP64 pipe bounds the passes, an idle owner's lane costs its full share
+// of it, and the two radices of these edges leave most of them idle (162 = 18 x 9:
+// eight threads take 24 and 16 owner slots), in the z pass for three components at
+// once.  FP64 apply, generic | specialised, us (x, y, z): 162^3 3186 | 3621, 64 x 162 x
+// 162 1162 | 1331, 200 x 200 x 162 4499 | 4976, 200^3 5550 | 5741, 216^3 6220 | 6692; on
+// the other side of the line 162 x 96 x 162 1847 | 1867, 100 x 216 x 216 3039 | 3004,
+// 162 x 162 x 32 828 | 665, 162 x 162 x 240 4734 | 4182, 192^3 3953 | 3803.
+inline bool fp64_generic_passes(int nx, int ny, int nz) {
+    auto slow = [](int n) { return n == 162 || n == 200 || n == 216; };
+    return slow(nz) && slow(ny) && (nz == 162 || slow(nx));
+}
+
 }  // namespace fp
