@@ -37,6 +37,7 @@
 
 #include "../../include/fftperm.h"
 #include "common.cuh"
+#include "conv_rules.h"
 #include "tma.cuh"
 
 #ifndef FP_TC_LBO
@@ -465,15 +466,6 @@ void ensure_smem_limit(K kern, std::atomic<unsigned long long>& done) {
     }
 }
 
-// shared memory of one CTA: barriers + its buffers, and at least the CTA's
-// share of the SM for its TMEM columns
-size_t tc_smem(int cin, int tile, int stages) {
-    const int ncols = tile < 32 ? 32 : tile;
-    const size_t need = 1024 + stages * ((size_t)kTcM * cin * 2 + (size_t)tile * cin * 2);
-    const size_t share = (size_t)233472 * ncols / 512;
-    return need > share ? need : share;
-}
-
 }  // namespace
 }  // namespace fp
 
@@ -493,15 +485,18 @@ extern "C" int fp_nn_conv_tc(int nx, int ny, int nz, int64_t total, int dilation
     if (blocks > 0x7fffffffLL) return FP_ERR_INVALID;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (cout != 16 && cout != 32 && cout != 64 && cout != 128) return FP_ERR_INVALID;
-    {
-        // The tile form takes dilation 1, up to 64 input channels (their rows and
-        // weights fit shared memory) and samples that 32-bit positions cover.  Its
-        // output channels are split until two CTAs fit an SM, or else one.
+    int dev = 0, sms = 152;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const fp::ConvCall call{nx, ny, nz, p.total / p.n, dilation, cin, cout, sms};
+    const fp::ConvPlan plan = fp::conv_plan(call);
+    const unsigned splits = (unsigned)(cout / plan.tile);
+    if (plan.halo) {
         fp::HaloConv h{};
         h.nx = nx;
         h.ny = ny;
         h.nz = nz;
-        h.samples = (int)(p.total / p.n);
+        h.samples = (int)call.samples;
         h.n = p.n;
         h.sign = sign;
         h.in = p.in;
@@ -512,70 +507,43 @@ extern "C" int fp_nn_conv_tc(int nx, int ny, int nz, int64_t total, int dilation
         h.relu = relu;
         h.out32 = p.out32;
         h.out16 = p.out16;
-        const long long pitch = nx + 2, plane = pitch * (ny + 2), vol = plane * nz;
-        const long long rows = fp::kTcM + 2 * (pitch + 1);
-        auto need = [&](int t) { return 1024 + (size_t)27 * t * cin * 2 + (size_t)3 * rows * cin * 2; };
-        int t = cout;
-        while (t > 16 && need(t) > 113 * 1024) t /= 2;
-        if (need(t) > 113 * 1024)
-            for (t = cout; t > 16 && need(t) > 226 * 1024;) t /= 2;
-        if (dilation == 1 && cin <= 64 && vol < (1LL << 30) && 3 * rows <= 0x3FFF && need(t) <= 226 * 1024 &&
-            p.total / p.n < (1LL << 30)) {
-            h.pitch = (int)pitch;
-            h.plane = (int)plane;
-            h.rows = (int)rows;
-            h.tiles = (int)((vol + fp::kTcM - 1) / fp::kTcM);
-            h.ntiles = (long long)h.tiles * h.samples;
-            const size_t share = (size_t)233472 * (t < 32 ? 32 : t) / 512;
-            const size_t hs = need(t) > share ? need(t) : share;
-            int dev = 0, sms = 152;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            const long long fit = std::min<long long>(16, 232448 / (long long)(hs + 1024));
-            const unsigned splits = (unsigned)(cout / t);
-            const unsigned gx = (unsigned)std::min<long long>(h.ntiles, std::max<long long>(1, fit * sms / splits));
+        h.pitch = nx + 2;
+        h.plane = (nx + 2) * (ny + 2);
+        h.rows = (int)fp::conv_halo_rows(nx);
+        h.ntiles = fp::conv_halo_tiles(call);
+        h.tiles = (int)(h.ntiles / h.samples);
+        const size_t smem = fp::conv_halo_smem(nx, cin, plan.tile);
+        const unsigned gx = (unsigned)fp::conv_halo_grid(call, plan.tile);
 #define FP_HALO_LAUNCH(C)                                                                \
     {                                                                                    \
         static std::atomic<unsigned long long> done_{0};                                 \
         fp::ensure_smem_limit(fp::k_conv_halo<C>, done_);                                \
         FP_LAUNCHED();                                                                   \
-        fp::k_conv_halo<C><<<dim3(gx, splits), fp::kTcThreads, hs, s>>>(h);              \
+        fp::k_conv_halo<C><<<dim3(gx, splits), fp::kTcThreads, smem, s>>>(h);            \
     }
-            switch (t) {
-                case 16: FP_HALO_LAUNCH(16) break;
-                case 32: FP_HALO_LAUNCH(32) break;
-                case 64: FP_HALO_LAUNCH(64) break;
-                default: FP_HALO_LAUNCH(128) break;
-            }
-#undef FP_HALO_LAUNCH
-            return cudaGetLastError() == cudaSuccess ? FP_OK : FP_ERR_CUDA;
+        switch (plan.tile) {
+            case 16: FP_HALO_LAUNCH(16) break;
+            case 32: FP_HALO_LAUNCH(32) break;
+            case 64: FP_HALO_LAUNCH(64) break;
+            default: FP_HALO_LAUNCH(128) break;
         }
+#undef FP_HALO_LAUNCH
+        return cudaGetLastError() == cudaSuccess ? FP_OK : FP_ERR_CUDA;
     }
-    // Output channels per CTA: all of them (the gathered rows serve them all)
-    // while the voxels alone give two CTAs per SM; fewer voxels, as on the
-    // coarse levels, split the channels down to 32.
-    int tile = cout;
-    while (tile > 32 && blocks * (cout / tile) < 304) tile /= 2;
-    // Four buffers where several CTAs still fit an SM (48 KB), else three.
-    const int stages = fp::tc_smem(cin, tile, 4) <= 49152 ? 4 : 3;
-    const size_t smem = fp::tc_smem(cin, tile, stages);
-    if (smem > 232448) return FP_ERR_INVALID;
+    const size_t smem = fp::conv_tap_smem(cin, plan.tile, plan.stages);
 #define FP_TC_LAUNCH(C, S)                                                                        \
-    {                                                                                             \
+    case C * 10 + S: {                                                                            \
         static std::atomic<unsigned long long> done_{0};                                          \
         fp::ensure_smem_limit(fp::k_conv_tc<C, S>, done_);                                        \
         FP_LAUNCHED();                                                                            \
-        fp::k_conv_tc<C, S><<<dim3((unsigned)blocks, (unsigned)(cout / C)), fp::kTcThreads, smem, s>>>(p); \
-    }
-    switch (tile * 10 + stages) {
-        case 163: FP_TC_LAUNCH(16, 3) break;
-        case 164: FP_TC_LAUNCH(16, 4) break;
-        case 323: FP_TC_LAUNCH(32, 3) break;
-        case 324: FP_TC_LAUNCH(32, 4) break;
-        case 643: FP_TC_LAUNCH(64, 3) break;
-        case 644: FP_TC_LAUNCH(64, 4) break;
-        case 1283: FP_TC_LAUNCH(128, 3) break;
-        default: FP_TC_LAUNCH(128, 4) break;
+        fp::k_conv_tc<C, S><<<dim3((unsigned)blocks, splits), fp::kTcThreads, smem, s>>>(p);      \
+    } break;
+    switch (plan.tile * 10 + plan.stages) {
+        FP_TC_LAUNCH(16, 2) FP_TC_LAUNCH(16, 3) FP_TC_LAUNCH(16, 4)
+        FP_TC_LAUNCH(32, 2) FP_TC_LAUNCH(32, 3) FP_TC_LAUNCH(32, 4)
+        FP_TC_LAUNCH(64, 2) FP_TC_LAUNCH(64, 3) FP_TC_LAUNCH(64, 4)
+        FP_TC_LAUNCH(128, 2) FP_TC_LAUNCH(128, 3) FP_TC_LAUNCH(128, 4)
+        default: return FP_ERR_INVALID;
     }
 #undef FP_TC_LAUNCH
     return cudaGetLastError() == cudaSuccess ? FP_OK : FP_ERR_CUDA;
