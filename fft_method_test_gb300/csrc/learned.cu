@@ -477,7 +477,12 @@ extern "C" int fp_nn_wgrad(int nx, int ny, int nz, int64_t total, int dilation, 
 extern "C" int fp_nn_bias_grad(const void* dy_bf16, int64_t total, int cout, float* db, void* stream) {
     if (!dy_bf16 || !db || total <= 0 || cout <= 0) return FP_ERR_INVALID;
     const int pieces = cout / 8;
-    if (cout % 8 == 0 && (pieces & (pieces - 1)) == 0 && pieces <= 128 &&
+    // Few rows go to the kernel of one block per channel: the cluster's barriers
+    // alone take 9 us. Block per channel | cluster, us: 512 x 64 5.1 | 9.9, 4096 x 256
+    // 9.1 | 10.6, 12288 x 64 10.8 | 10.9, 24576 x 16 10.8 | 11.0; beyond, 4096 x 512
+    // 13.3 | 10.9, 16384 x 64 12.8 | 10.4, 32768 x 16 11.9 | 10.7.
+    const bool few_rows = (long long)total * cout <= 1280 * 1024 && total <= (cout >= 64 ? 12288 : 24576);
+    if (!few_rows && cout % 8 == 0 && (pieces & (pieces - 1)) == 0 && pieces <= 128 &&
         (reinterpret_cast<uintptr_t>(dy_bf16) & 15) == 0) {
         // as many blocks as have four reads per thread to do, at most a cluster of 16
         // (four 64^3 cells with 16 channels: 81 us with 8 blocks and four reads in
