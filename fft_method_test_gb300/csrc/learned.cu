@@ -14,17 +14,18 @@
 //            transposed per tap)
 //   wgrad    dW[tap][o][i] = sum_v dy[v][o] x[v + off(tap)][i]
 //            (per tap a GEMM over voxels, wgrad.cuh; k_wgrad below for output
-//            counts that are no multiple of 16 and unaligned tensors; partials
-//            reduced in a fixed order: deterministic)
+//            counts that are no multiple of 16, unaligned tensors and short
+//            chunks; partials reduced in a fixed order: deterministic)
 // Channel counts: inputs of a convolution a multiple of 16 (the MMA's k),
 // outputs a multiple of 8 (its n), at most 64.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include "../../include/fftperm.h"
+#include <algorithm>
 #include <cooperative_groups.h>
 
+#include "../../include/fftperm.h"
 #include "common.cuh"
 #include "launch_rules.h"
 #include "wgrad.cuh"
@@ -449,10 +450,18 @@ extern "C" int fp_nn_wgrad(int nx, int ny, int nz, int64_t total, int dilation, 
     auto x = static_cast<const __nv_bfloat16*>(x_bf16);
     const int co16 = (cout + 15) / 16 * 16;
     const fp::WgradArgs wa{nx, ny, nz, g.n, g.total, dilation, dy, cout, x, cin, (long long)chunk, partial, dw};
+    // Short chunks stay with the former kernel (one warp per chunk and tap): the ring's
+    // eight warps then have few steps each and a sum of eight accumulator blocks to
+    // form. Former | ring, us, four 32^3 cells: 64 -> 64 channels, chunk 64 1151 | 2059,
+    // 160 860 | 929, 192 826 | 801; 64 -> 32, 96 597 | 671, 128 533 | 543, 160 499 | 450;
+    // 32 -> 32, 64 579 | 591, 96 494 | 413; 16 -> 16, 16 1321 | 659.
+    const int block = std::min(64, co16) * std::min(64, cin);
+    const bool short_chunk = chunk < std::min(block / 16, 192);
     const bool covered = (co16 == 16 || co16 == 32 || (co16 == 64 && cin >= 32)) &&
                          (cin == 16 || cin == 32 || (cin == 64 && co16 >= 32));
-    if (covered && fp::wgrad_ring_ok(wa)) return fp::wgrad_ring(wa, s) == cudaSuccess ? FP_OK : FP_ERR_CUDA;
-    // other output counts and unaligned tensors
+    if (covered && !short_chunk && fp::wgrad_ring_ok(wa))
+        return fp::wgrad_ring(wa, s) == cudaSuccess ? FP_OK : FP_ERR_CUDA;
+    // other output counts, unaligned tensors and short chunks
     const dim3 grid((unsigned)nchunks, 27);
 #define FP_WG(C16, CI)                                                                  \
     do {                                                                                \
