@@ -143,15 +143,6 @@ __device__ __forceinline__ float2 cscale<float2>(float2 a, float s) {
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(make_float2(s, s))));
     return bits_f2(r);
 }
-template <typename T2>
-__device__ __forceinline__ T2 cconj(T2 a) {
-    return cmk<T2>(a.x, -a.y);
-}
-// multiply by sign*i:  (sign*i)*(x + iy) = -sign*y + i*sign*x
-template <int SIGN, typename T2>
-__device__ __forceinline__ T2 cmul_si(T2 a) {
-    return SIGN < 0 ? cmk<T2>(a.y, -a.x) : cmk<T2>(-a.y, a.x);
-}
 
 // a + sign*i*b and a - sign*i*b as two scalar additions: the rotated operand is
 // never formed (a packed addition would have to swap its halves first)

@@ -110,7 +110,6 @@ cudaError_t fast_plan(Problem& P, const ApplyArgs& aa, FastPlan<T>& pl) {
     a.ny = P.ny;
     a.nz = P.nz;
     a.nxh = P.nxh;
-    a.rs = P.rs;
     a.nh = fast::spec_elems(P.nx, P.ny, P.nz);
     a.nrows = P.nrows;
     a.n = P.n;

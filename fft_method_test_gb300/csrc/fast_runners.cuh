@@ -1,7 +1,8 @@
 // fast_runners.cuh -- launch runners of the specialised apply passes
 // (fft_fast.cuh), one Passes<T, N> per precision and grid edge, instantiated
-// by fast32.cu / fast64.cu (powers of two) and fast32n.cu / fast64n.cu (48,
-// 80, 96, 160) so that the four build in parallel.
+// by fast32.cu / fast64.cu (powers of two), fast32n.cu / fast64n.cu (48, 80, 96,
+// 160) and fast_{s,m,l}{32,64}.cu (the edges of fft_edges.cuh) so that the ten
+// build in parallel.
 #pragma once
 
 #include <atomic>

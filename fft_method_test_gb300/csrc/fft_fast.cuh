@@ -1,11 +1,12 @@
-// fft_fast.cuh -- the five apply passes specialised at compile time for the
-// cubic grid edges 32, 48, 64, 80, 96, 128, 160 and 256, for compact-vector
-// operator applies (scatter in, gather out).  The generic engine of
-// fft_passes.cuh serves every other edge, source and destination.
+// fft_fast.cuh -- the five apply passes specialised at compile time for 36 grid
+// edges (32, 48, 64, 80, 96, 128, 160, 256 and those of fft_edges.cuh; the three
+// edges of a grid may differ), for compact-vector operator applies (scatter in,
+// gather out).  The generic engine of fft_passes.cuh serves every other edge,
+// source and destination.
 //
-// Each line of length N = R1 * R2 is transformed by TPL threads (TPL divides
-// R1 and R2) with the four-step decomposition, one vector component per
-// thread:
+// Each line of length N = R1 * R2 is transformed by TPL threads with the
+// four-step decomposition, one vector component per thread (where TPL does not
+// divide a radix, a thread's last owner may be idle):
 //
 //   x[R2*i + a]  (i < R1, a < R2)
 //   stage A  threads owning a: DFT-R1 over i, times W_N^(S a k) -> Y[k][a]
@@ -373,7 +374,7 @@ __host__ __device__ constexpr int kx_tile() {
 
 struct FastArgs {
     int nx, ny, nz, nxh;
-    long long rs, nh, nrows, n;
+    long long nh, nrows, n;
     int ktl;        // log2 of the kx tile width
     long long kts;  // elements of one kx tile of a component
     const float2* tw32x;  // stage twiddles of the specialised edges (AxisPlan::fw32)
@@ -445,13 +446,6 @@ __device__ __forceinline__ const FastArgs& member_args(const FastArgs& a0, int m
     } else {
         return a0;
     }
-}
-
-// threads of the x passes for `rows` grid rows per tile: 3*rows/2 complex
-// lines of TPL threads, rounded up to whole warps
-template <int N>
-__host__ __device__ constexpr int x_threads(int rows) {
-    return ((3 * rows / 2 * Split<N>::TPL + 31) / 32) * 32;
 }
 
 // ---- two real lines in one complex line --------------------------------------
@@ -552,9 +546,9 @@ constexpr int kMaxXThreads = 384;
 // shared memory with warp barriers, and the half spectra leave the registers
 // for HBM directly (a store covers TPL neighbouring kx).  The two spectra are
 // stored times two; the inverse pass takes the factor back with its 1/N.
-// Against separating the spectra through shared memory: 49 -> 35 M warp
-// instructions, 80.3 -> 69.7 us at 256^3 FP32 under ncu; L1 and latency bound
-// it (DRAM at 33 %, 22 warps per SM).
+// Against separating the spectra through shared memory: 49 -> 37 M warp
+// instructions, 80.3 -> 63.0 us at 256^3 FP32 under ncu (tiles of four rows); L1
+// bounds it (75 % of its peak; DRAM at 41 %, 25 warps per SM).
 template <typename T, int N, bool GROUP>
 __global__ void __launch_bounds__(kMaxXThreads) k_fx_fwd(const __grid_constant__ FastArgs a0) {
     pdl_wait();
@@ -651,13 +645,14 @@ __global__ void __launch_bounds__(kMaxXThreads) k_fx_fwd(const __grid_constant__
 
 // ---- P5: C2R x + gather + partial sums -------------------------------------------
 
-// Persistent CTAs walk tiles of `rows` grid rows.  Bound by L1 and the latency
-// of its loads (DRAM at 37 %).  Each thread reads its part
-// of the two half spectra of a line straight from HBM (TPL neighbouring kx per
+// Persistent CTAs walk tiles of `rows` grid rows.  Bound by the latency of its
+// loads (L1 at 56 % of its peak, DRAM at 40 %, 23 warps per SM).  Each thread reads
+// its part of the two half spectra of a line straight from HBM (TPL neighbouring kx per
 // load), so shared memory holds the lines of the exchange only and several
 // CTAs per SM cover the latency of each other's loads.  Against the former
 // form (raw rows staged by cp.async, Hermitian halves read from shared memory):
-// 60 -> 33 M warp instructions, 82.8 -> 70.4 us at 256^3 FP32 under ncu.
+// 60 -> 35 M warp instructions at 256^3 FP32; 83.5 us under ncu with the last
+// block's sum of 1216 partial rows, which was a kernel of its own beside 82.8 us.
 template <typename T, int N, bool GROUP>
 __global__ void __launch_bounds__(kMaxXThreads) k_fx_inv(const __grid_constant__ FastArgs a0) {
     pdl_wait();
@@ -833,8 +828,10 @@ __host__ __device__ constexpr size_t z_stage_bytes() {
 // Persistent CTAs walk the (kx tile, ky) tiles; thread = column + TX *
 // (owner + TPL * comp).  One thread has the TMA engine bring the spectral
 // tile (three boxes of {2 TX reals, 1, nz}) and the Green tile (six boxes of
-// {TX, 1, nz}) into a stage, completing on that stage's mbarrier; boxes past
-// the last kx column read zeros.  With two stages the tiles of iteration
+// {TX, 1, nz}) into a stage, completing on that stage's mbarrier.  Past the
+// last kx column the Green boxes read zeros and the spectral boxes the padding
+// columns of the blocked layout, which nothing writes and only inactive threads
+// would read.  With two stages the tiles of iteration
 // i + 1 load while tile i is transformed (one CTA per SM); with one stage the
 // next tile loads after the current one is done, and three CTAs per SM (at
 // most 112 registers per thread) overlap one another instead.  The phases

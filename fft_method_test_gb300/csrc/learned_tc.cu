@@ -5,7 +5,8 @@
 // src/solver/MinresSolver.hpp:23, that nothing fills).
 //
 // Implicit GEMM, one CTA per 128 voxels (the MMA's M), in two forms: k_conv_halo
-// below (dilation 1, up to 64 input channels) and, for the rest, k_conv_tc:
+// below (dilation 1, up to 64 input channels) and k_conv_tc; conv_rules.h chooses
+// the form, the output channels of a CTA and k_conv_tc's buffers by size:
 //   y[v][o] = sum_tap sum_i x[v + sign*dil*off(tap)][i] W[tap][o][i]
 // Activations are channels-last BF16 [voxel][channel], weights BF16
 // [27][cout][cin] (the data gradient passes the per-tap transposed weights
@@ -18,11 +19,11 @@
 // cin/16 MMAs of 128 x cout x 16 per tap and commits them to the buffer's
 // mbarrier; the 128 threads meanwhile gather the rows of tap t + STAGES - 1, so
 // the latency of a gather is hidden by STAGES - 1 taps (128 -> 128 channels on
-// four 8^3 cells: 101 us waiting for each tap's rows, 52 with this and the split
-// output channels).  A grid of few
-// voxels splits the output channels over blockIdx.y.  The epilogue reads the accumulator rows back with tcgen05.ld
-// (warp w owns TMEM lanes 32w..32w+31 = voxel rows), adds the bias, applies
-// ReLU and stores FP32 and/or BF16.
+// four 8^3 cells: 77 us with two buffers and all channels in a CTA, 48 with four
+// and sixteen channels).  A grid of few voxels splits the output channels over
+// blockIdx.y.  The epilogue reads the accumulator rows back with tcgen05.ld (warp w
+// owns TMEM lanes 32w..32w+31 = voxel rows), adds the bias, applies ReLU and
+// stores FP32 and/or BF16.
 //
 // Every wait is bounded (the mbarrier helpers of tma.cuh): on a timeout the
 // CTA raises the file-scope error flag (fp_nn_tc_error), frees its TMEM and

@@ -55,7 +55,8 @@ typedef struct fp_solver_stats {
     double final_rel_residual; /* SolverResult::final_rel_residual */
     int32_t converged;         /* SolverResult::converged          */
     int32_t refinements;       /* mixed precision: outer refinement steps taken */
-    double seconds;            /* wall time of the call            */
+    double seconds;            /* wall time of the solve; of all that iterate together in a block or
+                                * group, a third of that in fp_solve_permeability's lockstep */
 } fp_solver_stats;
 
 /* Replaces the GreenOperator constructor + IFFTBackend::initialize
