@@ -8,10 +8,10 @@
 // each take one group at a time (its own stream) and solve it with
 // fp_group_solve_permeability (one lockstep MINRES per load case over the
 // group, one launch per pass for all members) or, for a group of one, with
-// fp_solve_permeability, whose MINRES iterations are replayed as CUDA graphs
-// of 40.  The threads' kernels overlap on the GPU, so the small grids of a
-// batch fill the 152 SMs together.  Groups are taken largest first, which
-// keeps the tail of the batch short.
+// fp_solve_permeability (the three load cases in lockstep up to 160^3, else one
+// after another, their iterations replayed as CUDA graphs).  The threads' kernels
+// overlap on the GPU, so the small grids of a batch fill the 152 SMs together.
+// Groups are taken largest first, which keeps the tail of the batch short.
 //
 // Autotuner.  The y and z passes take `tile` kx columns per CTA and have a
 // TMA-fed and a register-fed variant; the inverse x pass has a bulk-copy

@@ -23,8 +23,10 @@ extern thread_local long long g_thread_launches;
 // and its writes are visible.  Their launch and block start-up overlap the end
 // of the kernel before; with pdl_trigger() near the end of a block's work the
 // next kernel's blocks are placed that much earlier.  Measured per mixed apply
-// (five launches): 48^3 28.7 -> 16.5 us, 64^3 30.4 -> 20.2, 96^3 47.7 -> 37.9,
-// 128^3 74.9 -> 63.3, 256^3 431 -> 422.
+// with its reduction to alpha (fp_time_apply, without | with the launch attribute):
+// 48^3 28.7 | 17.4 us, 64^3 30.8 | 21.9, 96^3 55.2 | 45.1, 128^3 76.4 | 65.2, 256^3
+// 456 | 443.  (A caller who launches one apply at a time waits for the host: 40 us
+// at 48^3 either way.)
 // Only the FP32 forward x, y and z passes trigger.  A kernel whose successor is
 // bound by the FP64 pipe must not: blocks placed while other blocks still run
 // go to the SMs that have room, and the fullest SM's pipe sets the time (FP64
